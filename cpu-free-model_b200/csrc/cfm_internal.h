@@ -33,9 +33,10 @@ int current_device_info(DeviceInfo *out);
 
 // Device-side state of one grid barrier; see barrier.cuh.
 struct BarrierState {
-    // count (low) and gen (high) are updated as one 64-bit word
-    unsigned int count;   // arrivals in the current generation
-    unsigned int gen;     // generation, bumped by the last arrival
+    // one 64-bit count of arrivals since the barrier was set to zero: count the low, gen
+    // the high half
+    unsigned int count;
+    unsigned int gen;
     int error;            // set to 1 by a wait that ran out of budget
     int where;            // barrier index at which the first timeout happened
     unsigned long long timeout_ns;

@@ -379,10 +379,6 @@ __global__ void __launch_bounds__(32 * TY, 4) j3d_sweeps_kernel(T *g0, T *g1, in
 // so block 0's upper halo is the last block's last row).  Synchronisation is
 // point-to-point: a per-block sweep counter, bounded waits on the two
 // neighbours only, no grid-wide barrier.
-__device__ __forceinline__ void st_release_u32(unsigned int *p, unsigned int v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 template <typename T, bool MIRROR>
 __global__ void __launch_bounds__(1024, 1)
     j2d_resident_kernel(const T *in, T *final_out, int nx, int ny, int niter, T *xbuf,
