@@ -26,6 +26,7 @@
 
 #include "barrier.cuh"
 #include "cfm_internal.h"
+#include "j2d_temporal.cuh"
 #include "j3d_tma.cuh"
 #include "j3d_tma2.cuh"
 #include "tma.cuh"
@@ -368,272 +369,6 @@ __global__ void __launch_bounds__(32 * TY, 4) j3d_sweeps_kernel(T *g0, T *g1, in
     }
 }
 
-// ---------------------------------------------------------- 2D resident sweep
-// PERKS-style temporal residency (the design of Stencil/jacobi2D/PERKS/
-// jacobi-general-kernel.cuh:22-505, re-derived): block b owns the interior
-// rows [r0, r1) and keeps them, plus one halo row above and below, in shared
-// memory for all sweeps (two copies, ping-pong).  Per sweep the only global
-// traffic is the block's first and last new rows, published to a
-// double-buffered exchange area, and its two halo rows read back from the
-// ring neighbours (b-1, b+1 mod B; the ring closes through the periodic rows,
-// so block 0's upper halo is the last block's last row).  Synchronisation is
-// point-to-point: a per-block sweep counter, bounded waits on the two
-// neighbours only, no grid-wide barrier.
-template <typename T, bool MIRROR>
-__global__ void __launch_bounds__(1024, 1)
-    j2d_resident_kernel(const T *in, T *final_out, int nx, int ny, int niter, T *xbuf,
-                        unsigned int *flags, BarrierState *bar) {
-    extern __shared__ __align__(16) unsigned char j2d_smem[];
-    const int B = gridDim.x, b = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
-    const int nrows = ny - 2;
-    const int r0 = 1 + (int)((long long)b * nrows / B);
-    const int r1 = 1 + (int)((long long)(b + 1) * nrows / B);
-    const int h = r1 - r0;
-    const int up_blk = (b + B - 1) % B, dn_blk = (b + 1) % B;
-    const size_t band = (size_t)(h + 2) * nx;
-    T *cur = reinterpret_cast<T *>(j2d_smem);
-    T *nxt = cur + band;
-    for (size_t i = tid; i < band; i += nth) {
-        const T v = in[(size_t)(r0 - 1) * nx + i];
-        cur[i] = v;
-        nxt[i] = v;
-    }
-    __syncthreads();
-    __shared__ int s_ok;
-    // updated columns: 1 .. nx-2, or with the mirror boundary 0 .. nx-1
-    const int x0 = MIRROR ? 0 : 1;
-    const int inner = MIRROR ? nx : nx - 2;
-    // rows [ra, rb) of the band as a flat run of cells, row r / column x of
-    // the first cell of each thread stepped without a division per cell
-    const int dr = nth / inner, dx = nth % inner;
-    auto sweep_rows = [&](int ra, int rb, T *pub) {
-        int r = ra + tid / inner, x = x0 + tid % inner;
-        for (; r < rb; r += dr, x += dx) {
-            if (x >= x0 + inner) {
-                x -= inner;
-                ++r;
-                if (r >= rb) break;
-            }
-            const T *c = cur + (size_t)r * nx + x;
-            T v;
-            if (MIRROR)  // Stencil/jacobi2D/src/common.cu:57-63
-                v = quarter<T>(add_rn(add_rn(add_rn(c[nx], c[-nx]), c[x < nx - 1 ? 1 : 0]),
-                                      c[x > 0 ? -1 : 0]));
-            else
-                v = quarter<T>(add_rn(add_rn(add_rn(c[1], c[-1]), c[nx]), c[-nx]));
-            nxt[(size_t)r * nx + x] = v;
-            if (pub) {  // the rows the neighbours read: first to slot 0, last to slot 1
-                if (r == 1) __stcg(pub + x, v);
-                if (r == h) __stcg(pub + nx + x, v);
-            }
-        }
-    };
-    for (int t = 0; t < niter; ++t) {
-        T *xb = xbuf + ((size_t)(t & 1) * B + b) * 2 * nx;
-        // 1. the first and last rows, published as they are computed (a
-        //    one-row band publishes its row in both slots)
-        sweep_rows(1, 2, xb);
-        if (h > 1) sweep_rows(h, h + 1, xb);
-        // the slot columns 0 and nx-1 carry the band's boundary cells
-        if (!MIRROR && tid == 0) {  // (mirror: sweep_rows published them)
-            __stcg(xb, nxt[nx]);
-            __stcg(xb + nx - 1, nxt[2 * (size_t)nx - 1]);
-            __stcg(xb + nx, nxt[(size_t)h * nx]);
-            __stcg(xb + 2 * nx - 1, nxt[(size_t)(h + 1) * nx - 1]);
-        }
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            st_release_u32(flags + b, (unsigned)(t + 1));
-        }
-        // 2. the inner rows while the neighbours' counters move
-        if (h > 2) sweep_rows(2, h, nullptr);
-        // 3. wait for the two ring neighbours' rows of this sweep
-        if (tid == 0) {
-            int ok = 1;
-            const unsigned long long t0 = global_ns();
-            const unsigned long long budget = bar->timeout_ns;
-            while (ld_acquire_u32(flags + up_blk) < (unsigned)(t + 1) ||
-                   ld_acquire_u32(flags + dn_blk) < (unsigned)(t + 1)) {
-                if (ld_relaxed_i32(&bar->error)) {
-                    ok = 0;
-                    break;
-                }
-                if (global_ns() - t0 > budget) {
-                    if (atomicCAS(&bar->error, 0, 1) == 0) bar->where = t;
-                    ok = 0;
-                    break;
-                }
-            }
-            __threadfence();
-            s_ok = ok;
-        }
-        __syncthreads();
-        if (!s_ok) return;
-        const T *up = xbuf + ((size_t)(t & 1) * B + up_blk) * 2 * nx + nx;  // last row above
-        const T *dn = xbuf + ((size_t)(t & 1) * B + dn_blk) * 2 * nx;       // first row below
-        for (int x = tid; x < nx; x += nth) {
-            nxt[x] = __ldcg(up + x);
-            nxt[(size_t)(h + 1) * nx + x] = __ldcg(dn + x);
-        }
-        __syncthreads();
-        T *tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-    }
-    // write the band back; the owners of rows 1 and ny-2 also write their
-    // periodic images (full rows, so the corner cells become images too)
-    for (size_t i = tid; i < (size_t)h * nx; i += nth) final_out[(size_t)r0 * nx + i] = cur[nx + i];
-    if (r0 == 1)
-        for (int x = tid; x < nx; x += nth) final_out[(size_t)(ny - 1) * nx + x] = cur[nx + x];
-    if (r1 == ny - 1)
-        for (int x = tid; x < nx; x += nth) final_out[x] = cur[(size_t)h * nx + x];
-}
-
-// The resident kernel with two sweeps per exchange (halo two rows deep): the
-// band lives in shared memory with two halo rows on each side (h + 4 rows,
-// twice).  The first sweep runs alone (the initial halo rows need not be
-// periodic images yet) and ends with an exchange of the block's first two
-// and last two rows; from then on each period is sweep A over rows r0 - 1 ..
-// r1 (the extra row on each side computed from the deeper halo, with the
-// same inputs and arithmetic as the neighbour that owns it, so the same
-// bits) and sweep B over the block's own rows r0 .. r1 - 1, then one
-// exchange; an odd last sweep runs alone.  Half the neighbour handshakes of
-// j2d_resident_kernel for 2 / h more computed rows.  Needs h >= 2.
-template <typename T, bool MIRROR>
-__global__ void __launch_bounds__(1024, 1)
-    j2d_resident2_kernel(const T *in, T *final_out, int nx, int ny, int niter, T *xbuf,
-                         unsigned int *flags, BarrierState *bar) {
-    extern __shared__ __align__(16) unsigned char j2d_smem[];
-    const int B = gridDim.x, b = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
-    const int nrows = ny - 2;
-    const int r0 = 1 + (int)((long long)b * nrows / B);
-    const int r1 = 1 + (int)((long long)(b + 1) * nrows / B);
-    const int h = r1 - r0;  // >= 2
-    const int up_blk = (b + B - 1) % B, dn_blk = (b + 1) % B;
-    // local row l of the band is global row r0 - 2 + l; own rows are 2 .. h + 1
-    const size_t band = (size_t)(h + 4) * nx;
-    T *cur = reinterpret_cast<T *>(j2d_smem);
-    T *nxt = cur + band;
-    // initial rows r0 - 1 .. r1 (local 1 .. h + 2) in both copies
-    for (size_t i = tid; i < (size_t)(h + 2) * nx; i += nth) {
-        const T v = in[(size_t)(r0 - 1) * nx + i];
-        cur[nx + i] = v;
-        nxt[nx + i] = v;
-    }
-    __syncthreads();
-    __shared__ int s_ok;
-    const int x0 = MIRROR ? 0 : 1;
-    const int inner = MIRROR ? nx : nx - 2;
-    const int dr = nth / inner, dx = nth % inner;
-    // rows [ra, rb) (local) of dst from src
-    auto sweep_rows = [&](const T *src, T *dst, int ra, int rb) {
-        if (ra >= rb) return;
-        int r = ra + tid / inner, x = x0 + tid % inner;
-        for (; r < rb; r += dr, x += dx) {
-            if (x >= x0 + inner) {
-                x -= inner;
-                ++r;
-                if (r >= rb) break;
-            }
-            const T *c = src + (size_t)r * nx + x;
-            T v;
-            if (MIRROR)
-                v = quarter<T>(add_rn(add_rn(add_rn(c[nx], c[-nx]), c[x < nx - 1 ? 1 : 0]),
-                                      c[x > 0 ? -1 : 0]));
-            else
-                v = quarter<T>(add_rn(add_rn(add_rn(c[1], c[-1]), c[nx]), c[-nx]));
-            dst[(size_t)r * nx + x] = v;
-        }
-    };
-    // The block's own rows of one sweep src -> dst: first its two edge rows
-    // at each end, published (full rows) to exchange slot `e`; then, when
-    // `publish`, the block's counter; then the inner rows; then, when
-    // `publish`, the neighbours' rows into dst's halo rows.  Returns false
-    // when a wait ran out.
-    auto own_sweep = [&](const T *src, T *dst, unsigned e, bool publish) -> bool {
-        const int ea = min(4, h + 2), eb = max(ea, h);
-        sweep_rows(src, dst, 2, ea);
-        sweep_rows(src, dst, eb, h + 2);
-        if (!publish) {
-            sweep_rows(src, dst, ea, eb);
-            return true;
-        }
-        __syncthreads();
-        T *xb = xbuf + ((size_t)(e & 1) * B + b) * 4 * nx;  // first two, last two rows
-        for (int i = tid; i < 2 * nx; i += nth) {
-            __stcg(xb + i, dst[2 * (size_t)nx + i]);
-            __stcg(xb + 2 * nx + i, dst[(size_t)h * nx + i]);
-        }
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            st_release_u32(flags + b, e);
-        }
-        sweep_rows(src, dst, ea, eb);
-        if (tid == 0) {
-            int ok = 1;
-            const unsigned long long t0 = global_ns();
-            const unsigned long long budget = bar->timeout_ns;
-            while (ld_acquire_u32(flags + up_blk) < e || ld_acquire_u32(flags + dn_blk) < e) {
-                if (ld_relaxed_i32(&bar->error)) {
-                    ok = 0;
-                    break;
-                }
-                if (global_ns() - t0 > budget) {
-                    if (atomicCAS(&bar->error, 0, 1) == 0) bar->where = (int)e;
-                    ok = 0;
-                    break;
-                }
-            }
-            __threadfence();
-            s_ok = ok;
-        }
-        __syncthreads();
-        if (!s_ok) return false;
-        const T *up = xbuf + ((size_t)(e & 1) * B + up_blk) * 4 * nx + 2 * nx;  // its last two rows
-        const T *dn = xbuf + ((size_t)(e & 1) * B + dn_blk) * 4 * nx;           // its first two rows
-        for (int i = tid; i < 2 * nx; i += nth) {
-            dst[i] = __ldcg(up + i);
-            dst[(size_t)(h + 2) * nx + i] = __ldcg(dn + i);
-        }
-        __syncthreads();
-        return true;
-    };
-    int t = 0;
-    unsigned e = 0;  // exchanges so far
-    if (niter > 0) {  // the first sweep alone, from the initial halo rows
-        if (!own_sweep(cur, nxt, ++e, niter > 1)) return;
-        T *tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-        t = 1;
-    }
-    while (t < niter) {
-        if (niter - t >= 2) {
-            sweep_rows(cur, nxt, 1, h + 3);  // sweep A: own rows and one more each side
-            __syncthreads();
-            if (!own_sweep(nxt, cur, ++e, t + 2 < niter)) return;  // sweep B, back into cur
-            t += 2;
-        } else {
-            if (!own_sweep(cur, nxt, ++e, false)) return;
-            __syncthreads();
-            T *tmp = cur;
-            cur = nxt;
-            nxt = tmp;
-            t += 1;
-        }
-    }
-    __syncthreads();
-    // write the band back; the owners of rows 1 and ny-2 also write their
-    // periodic images (full rows)
-    for (size_t i = tid; i < (size_t)h * nx; i += nth) final_out[(size_t)r0 * nx + i] = cur[2 * nx + i];
-    if (r0 == 1)
-        for (int x = tid; x < nx; x += nth) final_out[(size_t)(ny - 1) * nx + x] = cur[2 * nx + x];
-    if (r1 == ny - 1)
-        for (int x = tid; x < nx; x += nth) final_out[x] = cur[(size_t)(h + 1) * nx + x];
-}
-
 // Cells on the edges of the box (two or more coordinates on the boundary) are
 // neither read nor written by a sweep.  The reference's full-row/plane halo
 // copies leave each such cell equal to its periodic image after the first
@@ -722,6 +457,17 @@ struct TmaConfig {
 };
 }  // namespace cfm
 
+namespace cfm {
+// What the 2D persistent and resident runs of a handle launch.
+struct J2Plan {
+    const void *fn = nullptr;  // nullptr: not a 2D single-launch handle
+    bool tile = false;         // on chip, else streaming
+    J2Tiling tl{};
+    int blocks = 0, threads = 0, ts = 0;
+    size_t smem = 0;
+};
+}  // namespace cfm
+
 struct cfm_jacobi {
     cfm_jacobi_params p;
     size_t elems = 0, esize = 0;
@@ -733,13 +479,11 @@ struct cfm_jacobi {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int blocks = 0, threads = 0, zchunk = 0;
     int num_sms = 0;
-    // 2D resident kernel: exchange rows, per-block sweep counters, shape
-    void *xbuf = nullptr;
+    // 2D persistent and resident runs: the grid on chip (j2d_tile_kernel,
+    // with its blocks' exchange counters) or several sweeps per pass over it
+    // (j2d_stream_kernel)
+    cfm::J2Plan j2;
     unsigned int *flags = nullptr;
-    int res_blocks = 0;
-    size_t res_smem = 0;
-    bool res_two = false;  // two sweeps per exchange (j2d_resident2_kernel)
-    bool resident = false;
     // 3D TMA pipeline: the chosen shape, and (for a two-sweep shape) the
     // one-sweep shape that does the last sweep of an odd count
     bool tma = false;
@@ -989,19 +733,106 @@ const void *sweep_fn_any(const cfm_jacobi_params &p, bool images, bool mirror) {
                                    : sweep_fn<float>(p, images, mirror);
 }
 
-const void *resident_fn(const cfm_jacobi_params &p, bool mirror, bool two) {
-    if (two) {
-        if (p.precision == CFM_FP64)
-            return mirror ? (const void *)j2d_resident2_kernel<double, true>
-                          : (const void *)j2d_resident2_kernel<double, false>;
-        return mirror ? (const void *)j2d_resident2_kernel<float, true>
-                      : (const void *)j2d_resident2_kernel<float, false>;
+// Tile shapes of j2d_tile_kernel: rows per warp and warps per block.
+struct J2TileShape {
+    int rows, warps;
+    const void *fn[2];  // [mirror]
+    size_t smem;
+};
+template <typename T, int R, int WARPS>
+J2TileShape j2_tile_shape() {
+    return {R, WARPS, {(const void *)j2d_tile_kernel<T, R, WARPS, false>,
+                       (const void *)j2d_tile_kernel<T, R, WARPS, true>}, j2_tile_smem<T, WARPS>()};
+}
+const std::vector<J2TileShape> &j2_tile_shapes(int precision) {
+    static const std::vector<J2TileShape> f64 = {
+        j2_tile_shape<double, 2, 32>(), j2_tile_shape<double, 3, 32>(), j2_tile_shape<double, 4, 32>(),
+        j2_tile_shape<double, 4, 16>(), j2_tile_shape<double, 6, 16>(), j2_tile_shape<double, 7, 16>()};
+    static const std::vector<J2TileShape> f32 = {
+        j2_tile_shape<float, 2, 32>(), j2_tile_shape<float, 3, 32>(), j2_tile_shape<float, 4, 32>(),
+        j2_tile_shape<float, 3, 16>(), j2_tile_shape<float, 4, 16>(), j2_tile_shape<float, 6, 16>(),
+        j2_tile_shape<float, 8, 16>(), j2_tile_shape<float, 12, 16>()};
+    return precision == CFM_FP64 ? f64 : f32;
+}
+
+// Tiles of `rows` window rows with K sweeps per exchange that cover an nx x ny
+// grid with at most `blocks` blocks: every block must own at least K rows and
+// (with neighbours in x) K columns, since its rim comes from the adjacent blocks.
+bool j2_tiling(int nx, int ny, int rows, int K, int blocks, J2Tiling *t) {
+    const int P = ny - 2, hu = rows - 2 * K, wu = J2T_W - 2 * K;
+    if (hu < K || wu < K) return false;
+    t->k = K;
+    t->ty = (P + hu - 1) / hu;
+    if (P / t->ty < K) return false;
+    t->tx = 1;
+    t->ux = J2T_W;
+    if (nx > J2T_W) {
+        t->tx = std::max(2, (nx - 2 * K + wu - 1) / wu);
+        t->ux = ((nx - 2 * K + t->tx - 1) / t->tx + J2T_V - 1) / J2T_V * J2T_V;
+        const int last = nx - (K + (t->tx - 1) * t->ux);
+        if (t->ux < K || last < K || last > wu + K) return false;
     }
-    if (p.precision == CFM_FP64)
-        return mirror ? (const void *)j2d_resident_kernel<double, true>
-                      : (const void *)j2d_resident_kernel<double, false>;
-    return mirror ? (const void *)j2d_resident_kernel<float, true>
-                  : (const void *)j2d_resident_kernel<float, false>;
+    return (long long)t->tx * t->ty <= blocks;
+}
+
+// 2D persistent and resident runs: the grid on chip wherever a tiling covers it with
+// one block per SM, else the streaming kernel.  The tile shape and K are those with the
+// shortest modelled sweep, window rows x time per row + an exchange / K (fitted to B200
+// runs of 256^2 to 1500^2: 6.2 ns per 128-column row in FP32, 11.8 in FP64, 6% more with
+// 32 warps; 2.7 us per exchange).  On chip against streaming: 1024^2 FP64 1.5 against 2.9
+// us per sweep, 1500^2 FP32 1.5 against 3.0, 1100^2 FP64 with K = 4 (the least) 2.7
+// against 2.7.  Resident handles keep to blocks of 1024 threads where those cover the
+// grid (cfm_jacobi_launch_shape's sign of an on-chip run).
+int plan_j2(cfm_jacobi *h) {
+    const cfm_jacobi_params &p = h->p;
+    J2Plan best;
+    double best_cost = 1e300;
+    for (const J2TileShape &s : j2_tile_shapes(p.precision))
+        for (int K : {4, 8, 12, 16, 20, 24}) {
+            J2Tiling t;
+            if (!j2_tiling(p.nx, p.ny, s.rows * s.warps, K, h->num_sms, &t)) continue;
+            const double row = (p.precision == CFM_FP64 ? 0.0118 : 0.0062) * (s.warps == 32 ? 1.06 : 1.0);
+            double cost = row * s.rows * s.warps + 2.7 / K;
+            if (p.impl == CFM_JACOBI_RESIDENT && s.warps != 32) cost += 1e6;
+            if (cost >= best_cost) continue;
+            best_cost = cost;
+            best.fn = s.fn[h->mirror ? 1 : 0];
+            best.tile = true;
+            best.tl = t;
+            best.blocks = t.tx * t.ty;
+            best.threads = 32 * s.warps;
+            best.smem = s.smem;
+        }
+    if (!best.fn) {
+        best.threads = 32 * J2S_WARPS;
+        best.ts = J2S_SWEEPS;
+        const bool vec = p.nx % (16 / (int)h->esize) == 0;
+        auto pick = [&](auto t, auto v) {
+            using T = decltype(t);
+            constexpr int V = decltype(v)::value;
+            best.fn = h->mirror ? (vec ? (const void *)j2d_stream_kernel<T, V, J2S_SWEEPS, true, true>
+                                       : (const void *)j2d_stream_kernel<T, V, J2S_SWEEPS, true, false>)
+                                : (vec ? (const void *)j2d_stream_kernel<T, V, J2S_SWEEPS, false, true>
+                                       : (const void *)j2d_stream_kernel<T, V, J2S_SWEEPS, false, false>);
+            best.smem = (size_t)J2S_WARPS * J2S_D * 32 * V * sizeof(T);
+        };
+        if (p.precision == CFM_FP64)
+            pick(double(), std::integral_constant<int, 2>());
+        else
+            pick(float(), std::integral_constant<int, 4>());
+    }
+    CFM_CUDA_TRY(cudaFuncSetAttribute(best.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best.smem));
+    if (!best.tile) {
+        int per_sm = 0;
+        CFM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, best.fn, best.threads, best.smem));
+        if (per_sm < 1) {
+            set_error("sweep kernel cannot be resident");
+            return CFM_UNSUPPORTED;
+        }
+        best.blocks = per_sm * h->num_sms;
+    }
+    h->j2 = best;
+    return CFM_OK;
 }
 
 dim3 block_of(const cfm_jacobi_params &p) { return p.dims == 2 ? dim3(256) : dim3(32, J3_TY); }
@@ -1077,31 +908,8 @@ int choose_launch(cfm_jacobi *h) {
         const long long need = (units * 32 + threads - 1) / threads;
         if (need < h->blocks) h->blocks = (int)std::max(1LL, need);
     }
-    if (p.dims == 2 && p.impl == CFM_JACOBI_RESIDENT) {
-        // One 1024-thread block per SM, each holding its band twice in shared
-        // memory; used only when that fits on chip.  Preferred: two sweeps
-        // per exchange (bands of >= 2 rows plus 2 halo rows each side), else
-        // one (any band, 1 halo row each side).
-        h->resident = false;
-        for (int two = 1; two >= 0 && !h->resident; --two) {
-            const int B = std::min(di.num_sms, two ? (p.ny - 2) / 2 : p.ny - 2);
-            if (B < 1) continue;
-            const int hmax = (p.ny - 2 + B - 1) / B;
-            const size_t smem = 2 * (size_t)(hmax + (two ? 4 : 2)) * p.nx * h->esize;
-            const void *rfn = resident_fn(p, h->mirror, two != 0);
-            if (smem > di.smem_optin) continue;
-            CFM_CUDA_TRY(cudaFuncSetAttribute(rfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
-            int rper = 0;
-            CFM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rper, rfn, 1024, smem));
-            if (rper >= 1) {
-                h->resident = true;
-                h->res_two = two != 0;
-                h->res_blocks = B;
-                h->res_smem = smem;
-            }
-        }
-    }
+    if (p.dims == 2 && (p.impl == CFM_JACOBI_PERSISTENT || p.impl == CFM_JACOBI_RESIDENT))
+        return plan_j2(h);
     return CFM_OK;
 }
 
@@ -1180,18 +988,22 @@ int host_loop_images(cfm_jacobi *h, int niter, int *launches) {
     return CFM_OK;
 }
 
-int resident2d(cfm_jacobi *h, int niter, int *launches) {
+int launch_j2(cfm_jacobi *h, int niter, int *launches) {
     const cfm_jacobi_params &p = h->p;
-    CFM_CUDA_TRY(cudaMemsetAsync(h->flags, 0, sizeof(unsigned int) * h->res_blocks, h->stream));
-    const void *in = h->buf[h->cur];
-    void *fin = h->buf[h->cur ^ (niter & 1)];
-    int n = niter;
-    void *args[] = {(void *)&in, &fin, (void *)&p.nx, (void *)&p.ny, &n, &h->xbuf, &h->flags,
-                    &h->bar};
-    const void *fn = resident_fn(p, h->mirror, h->res_two);
-    CFM_CUDA_TRY(launch_cooperative(fn, dim3(h->res_blocks), dim3(1024), args, h->res_smem,
-                                    h->stream));
-    h->cur ^= (niter & 1);
+    J2Plan &pl = h->j2;
+    void *in = h->buf[h->cur], *out = h->buf[h->cur ^ 1];
+    int n = niter, swaps;
+    if (pl.tile) {
+        CFM_CUDA_TRY(cudaMemsetAsync(h->flags, 0, sizeof(unsigned int) * pl.blocks, h->stream));
+        void *args[] = {&in, &out, (void *)&p.nx, (void *)&p.ny, &n, &pl.tl, &h->flags, &h->bar};
+        CFM_CUDA_TRY(launch_cooperative(pl.fn, dim3(pl.blocks), dim3(pl.threads), args, pl.smem, h->stream));
+        swaps = (niter - 1 + pl.tl.k - 1) / pl.tl.k + 1;  // exchanges after the first sweep, and the result
+    } else {
+        void *args[] = {&in, &out, (void *)&p.nx, (void *)&p.ny, &n, &h->bar};
+        CFM_CUDA_TRY(launch_cooperative(pl.fn, dim3(pl.blocks), dim3(pl.threads), args, pl.smem, h->stream));
+        swaps = j2s_passes(niter, pl.ts);
+    }
+    h->cur ^= swaps & 1;
     ++*launches;
     return CFM_OK;
 }
@@ -1230,7 +1042,7 @@ int persistent_tma(cfm_jacobi *h, int niter, int *launches) {
 
 int persistent(cfm_jacobi *h, int niter, int *launches) {
     const cfm_jacobi_params &p = h->p;
-    if (h->resident) return resident2d(h, niter, launches);
+    if (h->j2.fn) return launch_j2(h, niter, launches);
     if (h->tma) return persistent_tma(h, niter, launches);
     const void *fn = sweep_fn_any(p, true, h->mirror);
     void *in = h->buf[h->cur], *out = h->buf[h->cur ^ 1];
@@ -1256,8 +1068,9 @@ int reset_barrier(cfm_jacobi *h) {
 int enqueue_sweeps(cfm_jacobi *h, int niter, int *launches) {
     if (niter == 0) return CFM_OK;
     int st;
-    // (the mirror sweep reads the edge cells and writes whole rows: no preset)
-    if (h->p.impl != CFM_JACOBI_HOST_LOOP && !h->mirror) {
+    // (the mirror sweep reads the edge cells and writes whole rows, and the 2D
+    // single-launch kernels write the whole grid: no preset)
+    if (h->p.impl != CFM_JACOBI_HOST_LOOP && !h->mirror && !h->j2.fn) {
         st = h->p.precision == CFM_FP64 ? launch_edge_preset<double>(h)
                                         : launch_edge_preset<float>(h);
         if (st) return st;
@@ -1361,14 +1174,10 @@ int cfm_jacobi_create(const cfm_jacobi_params *p, cfm_jacobi **out) {
     if ((st = choose_launch(h))) return fail(st);
     if (h->p.impl == CFM_JACOBI_PERSISTENT || h->p.impl == CFM_JACOBI_RESIDENT)
         if ((st = setup_tma(h, default_tma_variant()))) return fail(st);
-    if (h->resident) {
-        // exchange rows: 2 parities x blocks x 4 rows (the first and last two)
-        const size_t xbytes = 2 * (size_t)h->res_blocks * 4 * h->p.nx * h->esize;
-        if ((e = cudaMalloc(&h->xbuf, xbytes)) != cudaSuccess ||
-            (e = cudaMalloc(&h->flags, sizeof(unsigned int) * h->res_blocks)) != cudaSuccess) {
-            set_error("exchange buffers: %s", cudaGetErrorString(e));
-            return fail(CFM_CUDA_ERROR);
-        }
+    if (h->j2.fn &&
+        (e = cudaMalloc(&h->flags, sizeof(unsigned int) * h->num_sms)) != cudaSuccess) {
+        set_error("exchange counters: %s", cudaGetErrorString(e));
+        return fail(CFM_CUDA_ERROR);
     }
     // Zero both grids on the handle's own (non-blocking) stream: a legacy-
     // stream memset would not be ordered before later work on that stream.
@@ -1391,7 +1200,6 @@ void cfm_jacobi_destroy(cfm_jacobi *h) {
     for (int i = 0; i < 2; ++i)
         if (h->buf[i]) cudaFree(h->buf[i]);
     if (h->bar) cudaFree(h->bar);
-    if (h->xbuf) cudaFree(h->xbuf);
     if (h->flags) cudaFree(h->flags);
     if (h->udone) cudaFree(h->udone);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1616,9 +1424,9 @@ int cfm_jacobi_autotune(cfm_jacobi *h, int sweeps, int *best_variant, double *be
 int cfm_jacobi_launch_shape(cfm_jacobi *h, int *blocks, int *threads) {
     CFM_ARG_CHECK(h, "handle is null");
     int b = h->blocks, t = h->threads;
-    if (h->resident) {
-        b = h->res_blocks;
-        t = 1024;
+    if (h->j2.fn) {
+        b = h->j2.blocks;
+        t = h->j2.threads;
     } else if (h->tma) {
         b = h->tc.blocks;
         t = h->tc.threads;
