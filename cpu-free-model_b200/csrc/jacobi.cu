@@ -27,8 +27,8 @@
 #include "barrier.cuh"
 #include "cfm_internal.h"
 #include "j2d_temporal.cuh"
+#include "j3d_pair.cuh"
 #include "j3d_tma.cuh"
-#include "j3d_tma2.cuh"
 #include "tma.cuh"
 
 namespace cfm {
@@ -444,12 +444,11 @@ __global__ void load_problem_kernel(T *a, int dims, int nx, int ny, int nz, int 
 using namespace cfm;
 
 namespace cfm {
-// One configuration of the 3D TMA pipeline: tensor maps over both grids
-// (main boxes and, for two sweeps per pass, the 3-row far-row boxes), the
-// kernel and its launch shape.
+// One configuration of the 3D pipelines: the kernel and its launch shape, and for
+// the one-sweep TMA kernel tensor maps over both grids.
 struct TmaConfig {
     bool ok = false;
-    CUtensorMap map[2], xmap[2];
+    CUtensorMap map[2];
     const void *fn = nullptr;
     int var = 0, sweeps = 1, blocks = 0, zchunk = 0, threads = 0;
     long long units = 0;
@@ -484,8 +483,8 @@ struct cfm_jacobi {
     // (j2d_stream_kernel)
     cfm::J2Plan j2;
     unsigned int *flags = nullptr;
-    // 3D TMA pipeline: the chosen shape, and (for a two-sweep shape) the
-    // one-sweep shape that does the last sweep of an odd count
+    // 3D pipelines: the chosen shape, and beside a two-sweep shape the one-sweep
+    // shape of the neighbourhood order
     bool tma = false;
     cfm::TmaConfig tc, tail;
     size_t smem_optin = 0;
@@ -528,6 +527,24 @@ int pick_zchunk(long long ntiles, int nzi, int *blocks) {
     return best;
 }
 
+// The same for two sweeps per pass: every unit marches through four planes more than
+// its own.  All even splits of the planes are tried.
+int pick_pair_zchunk(long long ntiles, int nzi, int *blocks) {
+    int best = nzi;
+    long long best_cost = -1;
+    for (int n = 1; n <= nzi; ++n) {
+        const int zc = (nzi + n - 1) / n;
+        const long long rounds = (units_of(ntiles, nzi, zc) + *blocks - 1) / *blocks;
+        const long long cost = rounds * (zc + 4);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = zc;
+        }
+    }
+    *blocks = (int)std::min<long long>(*blocks, units_of(ntiles, nzi, best));
+    return best;
+}
+
 constexpr int J3_TY = 8;
 
 // Shapes of the TMA pipeline compiled into the library: consumer warps, rows
@@ -536,10 +553,11 @@ constexpr int J3_TY = 8;
 // CFM_J3D_TMA_VARIANT (an index into this table) overrides the choice.
 struct TmaVariant {
     int cw, rpw, stages;
-    int sweeps;            // sweeps per pass over the grid (2: j3d_tma2_kernel)
+    int sweeps;            // sweeps per pass over the grid (2: j3d_pair_kernel)
     const void *fn[2][2];  // [precision][periodic_y]
     size_t smem[2];        // [precision]
     int tx[2];             // [precision]
+    long long (*tiles)(int precision, int nx, int ny) = nullptr;  // two-sweep shapes
 };
 
 template <int CW, int RPW, int S>
@@ -556,17 +574,15 @@ TmaVariant make_tma_variant() {
     return v;
 }
 
-template <int CW, int RPW, int S>
-TmaVariant make_tma2_variant() {
-    TmaVariant v{CW, RPW, S, 2, {}, {}, {}};
-    v.fn[CFM_FP64][0] = (const void *)j3d_tma2_kernel<double, CW, RPW, S, false>;
-    v.fn[CFM_FP64][1] = (const void *)j3d_tma2_kernel<double, CW, RPW, S, true>;
-    v.fn[CFM_FP32][0] = (const void *)j3d_tma2_kernel<float, CW, RPW, S, false>;
-    v.fn[CFM_FP32][1] = (const void *)j3d_tma2_kernel<float, CW, RPW, S, true>;
-    v.smem[CFM_FP64] = Tma2Geom<double, CW, RPW, S>::SMEM;
-    v.smem[CFM_FP32] = Tma2Geom<float, CW, RPW, S>::SMEM;
-    v.tx[CFM_FP64] = Tma2Geom<double, CW, RPW, S>::TX;
-    v.tx[CFM_FP32] = Tma2Geom<float, CW, RPW, S>::TX;
+TmaVariant make_pair_variant(int i) {
+    const J3PairShape &p = j3d_pair_shape(i, true);
+    TmaVariant v{p.cw, p.rpw, p.stages, 2, {}, {}, {}};
+    for (int prec = 0; prec < 2; ++prec) {
+        for (int py = 0; py < 2; ++py) v.fn[prec][py] = p.fn[prec][py];
+        v.smem[prec] = p.smem;
+        v.tx[prec] = p.tx[prec];
+    }
+    v.tiles = p.tiles;
     return v;
 }
 
@@ -577,8 +593,7 @@ const TmaVariant *tma_variants(int *count) {
         make_tma_variant<8, 1, 8>(), make_tma_variant<4, 2, 12>(), make_tma_variant<2, 4, 8>(),
         make_tma_variant<8, 4, 4>(), make_tma_variant<16, 2, 4>(),  make_tma_variant<16, 2, 6>(),
         make_tma_variant<16, 2, 8>(), make_tma_variant<8, 4, 8>(),  make_tma_variant<16, 4, 4>(),
-        make_tma2_variant<16, 2, 4>(), make_tma2_variant<16, 2, 6>(), make_tma2_variant<8, 4, 5>(),
-        make_tma2_variant<8, 2, 4>(),
+        make_pair_variant(0), make_pair_variant(1), make_pair_variant(2), make_pair_variant(3),
     };
     *count = (int)(sizeof(v) / sizeof(v[0]));
     return v;
@@ -591,40 +606,39 @@ const TmaVariant &tma_variant(int i) {
 }
 
 
-// Tensor maps over both grids: dims (nx, ny, nz), box (TX + 2 VN, TY + 2, 1)
-// for one sweep per pass, (TX + 2 VN, TY + 4, 1) plus the 3-row far-row box
-// for two; zero fill outside.  Needs the row pitch nx * esize to be a
-// multiple of 16.  Leaves c->ok false when the pipeline does not apply.
+// The pipeline shape `var` for this handle: tensor maps over both grids, dims (nx, ny,
+// nz), box (TX + 2 VN, TY + 2, 1) for one sweep per pass, (TX, TY, 1) for two, zero fill
+// outside.  The row pitch nx * esize has to be a multiple of 16 for one sweep; two take
+// any row length (no maps then).  Leaves c->ok false when the shape does not apply.
 int build_tma(cfm_jacobi *h, int var, int zchunk, TmaConfig *c) {
     const cfm_jacobi_params &p = h->p;
     c->ok = false;
-    if (p.dims != 3 || ((size_t)p.nx * h->esize) % 16 != 0) return CFM_OK;
-    auto enc = tensor_map_encoder();
-    if (!enc) return CFM_OK;
+    if (p.dims != 3) return CFM_OK;
+    const bool two = tma_variant(var).sweeps == 2;
+    if (!two && ((size_t)p.nx * h->esize) % 16 != 0) return CFM_OK;
+    const bool maps = ((size_t)p.nx * h->esize) % 16 == 0;  // (the two-sweep kernel can do without)
+    auto enc = maps ? tensor_map_encoder() : nullptr;
+    if (maps && !enc) return CFM_OK;
     const TmaVariant &V = tma_variant(var);
     const int ty = V.cw * V.rpw, tx = V.tx[p.precision];
     const int vn = (int)(16 / h->esize);
     const cuuint64_t dims[3] = {(cuuint64_t)p.nx, (cuuint64_t)p.ny, (cuuint64_t)p.nz};
     const cuuint64_t strides[2] = {(cuuint64_t)p.nx * h->esize, (cuuint64_t)p.nx * p.ny * h->esize};
-    const cuuint32_t box[3] = {(cuuint32_t)(tx + 2 * vn), (cuuint32_t)(ty + (V.sweeps == 2 ? 4 : 2)), 1u};
-    const cuuint32_t xbox[3] = {(cuuint32_t)(tx + 2 * vn), 3u, 1u};
+    const cuuint32_t box[3] = {(cuuint32_t)(two ? tx : tx + 2 * vn), (cuuint32_t)(two ? ty : ty + 2), 1u};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType dt =
         p.precision == CFM_FP64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < 2 && maps; ++i) {
         CUresult r = enc(&c->map[i], dt, 3, h->buf[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r == CUDA_SUCCESS && V.sweeps == 2)
-            r = enc(&c->xmap[i], dt, 3, h->buf[i], dims, strides, xbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return CFM_OK;  // stay on the register kernel
     }
-    const void *fn = V.fn[p.precision][p.periodic_y ? 1 : 0];
-    const size_t smem = V.smem[p.precision];
+    const J3PairShape *ragged = two && !maps ? &j3d_pair_shape(0, false) : nullptr;
+    const void *fn = (ragged ? ragged->fn : V.fn)[p.precision][p.periodic_y ? 1 : 0];
+    const size_t smem = ragged ? ragged->smem : V.smem[p.precision];
     if (smem > h->smem_optin) return CFM_OK;
-    const int threads = 32 * (V.cw + 1);
+    const int threads = 32 * ((ragged ? ragged->cw : V.cw) + 1);
     CFM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // all of the SM's shared memory for the ring (two rings per SM when they fit)
     CFM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -633,7 +647,8 @@ int build_tma(cfm_jacobi *h, int var, int zchunk, TmaConfig *c) {
     CFM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
     if (per_sm < 1) return CFM_OK;
     c->blocks = per_sm * h->num_sms;
-    const long long ntiles = (long long)((p.nx + tx - 1) / tx) * ((p.ny - 2 + ty - 1) / ty);
+    const long long ntiles = two ? (ragged ? ragged->tiles : V.tiles)(p.precision, p.nx, p.ny)
+                                 : (long long)((p.nx + tx - 1) / tx) * ((p.ny - 2 + ty - 1) / ty);
     if (zchunk <= 0)
         if (const char *zc = std::getenv("CFM_J3D_ZCHUNK")) zchunk = std::atoi(zc);
     if (zchunk >= 1) {
@@ -641,7 +656,8 @@ int build_tma(cfm_jacobi *h, int var, int zchunk, TmaConfig *c) {
         const long long U = units_of(ntiles, p.nz - 2, c->zchunk);
         if (U < c->blocks) c->blocks = (int)std::max(1LL, U);
     } else {
-        c->zchunk = pick_zchunk(ntiles, p.nz - 2, &c->blocks);
+        c->zchunk = two ? pick_pair_zchunk(ntiles, p.nz - 2, &c->blocks)
+                        : pick_zchunk(ntiles, p.nz - 2, &c->blocks);
     }
     // one completion counter per unit for the neighbourhood-ordered sweeps
     const long long U = units_of(ntiles, p.nz - 2, c->zchunk);
@@ -665,32 +681,35 @@ int build_tma(cfm_jacobi *h, int var, int zchunk, TmaConfig *c) {
     return CFM_OK;
 }
 
-int default_tma_variant();
-
-// The pipeline shape `var` (and, for two sweeps per pass, the default
-// one-sweep shape for the last sweep of an odd count).
+// The pipeline shape `var` and, beside a two-sweep one, the default one-sweep shape
+// that the neighbourhood order of the sweeps (cfm_jacobi_set_dataflow) runs on.
 int setup_tma(cfm_jacobi *h, int var, int zchunk = 0) {
     h->tma = false;
+    h->tail.ok = false;
     int st = build_tma(h, var, zchunk, &h->tc);
     if (st || !h->tc.ok) return st;
-    if (h->tc.sweeps == 2) {
-        int dv = default_tma_variant();
-        if (tma_variant(dv).sweeps != 1) dv = 0;
-        if ((st = build_tma(h, dv, 0, &h->tail))) return st;
-        if (!h->tail.ok) return CFM_OK;
-    }
+    if (h->tc.sweeps == 2 && (st = build_tma(h, 0, 0, &h->tail))) return st;
     h->tma = true;
     return CFM_OK;
 }
 
-int default_tma_variant() {
+// Two sweeps per pass (shape 12) where the two grids are beyond L2, or so small that the
+// passes' latency and barriers are most of a sweep; between, one sweep per pass (shape
+// 0), which has no overlap to compute twice and runs from L2.  100 sweeps on B200, two
+// against one: 512^3 FP64 29.1 / 41 ms, 256^3 FP64 (268 MB) 5.2 / 5.1, 256^3 FP32 (134 MB) 3.8
+// / 3.25, 192^3 FP64 (113 MB) 2.5 / 2.3, 128^3 FP64 (34 MB) 1.06 / 0.86, 128^3 FP32 (17 MB) 0.66
+// / 0.82, 64^3 FP64 0.46 / 0.77.  Rows that are not a multiple of 16 bytes have no
+// one-sweep shape.  CFM_J3D_TMA_VARIANT (an index into the table) overrides.
+int default_tma_variant(const cfm_jacobi *h) {
     int n = 0;
     tma_variants(&n);
     if (const char *e = std::getenv("CFM_J3D_TMA_VARIANT")) {
         const int v = std::atoi(e);
         if (v >= 0 && v < n) return v;
     }
-    return 0;
+    const double bytes = 2.0 * (double)h->elems * (double)h->esize;
+    const bool whole = ((size_t)h->p.nx * h->esize) % 16 == 0;
+    return whole && bytes >= 20e6 && bytes < 250e6 ? 0 : 12;
 }
 
 int check_params(const cfm_jacobi_params *p) {
@@ -1015,9 +1034,12 @@ int launch_tma(cfm_jacobi *h, const TmaConfig &c, int count, int *launches) {
     void *g0 = h->buf[cu], *g1 = h->buf[cu ^ 1];
     int n = count, zc = c.zchunk;
     if (c.sweeps == 2) {
-        void *args[] = {(void *)&c.map[cu], (void *)&c.map[cu ^ 1], (void *)&c.xmap[cu], (void *)&c.xmap[cu ^ 1],
-                        &g0, &g1, (void *)&p.nx, (void *)&p.ny, (void *)&p.nz, &n, &zc, &h->bar};
+        void *args[] = {(void *)&c.map[cu], (void *)&c.map[cu ^ 1], &g0, &g1, (void *)&p.nx, (void *)&p.ny,
+                        (void *)&p.nz, &n, &zc, &h->bar};
         CFM_CUDA_TRY(launch_cooperative(c.fn, dim3(c.blocks), dim3(c.threads), args, c.smem, h->stream));
+        h->cur ^= j3p_passes(count) & 1;
+        ++*launches;
+        return CFM_OK;
     } else {
         unsigned int *ud = h->dataflow && count > 1 ? h->udone : nullptr;
         if (ud) CFM_CUDA_TRY(cudaMemsetAsync(ud, 0, sizeof(unsigned int) * c.units, h->stream));
@@ -1030,14 +1052,9 @@ int launch_tma(cfm_jacobi *h, const TmaConfig &c, int count, int *launches) {
     return CFM_OK;
 }
 
-// niter sweeps: one launch, or for two sweeps per pass niter / 2 passes and,
-// for an odd count, one more launch of the one-sweep shape.
 int persistent_tma(cfm_jacobi *h, int niter, int *launches) {
-    if (h->tc.sweeps == 1) return launch_tma(h, h->tc, niter, launches);
-    int st = CFM_OK;
-    if (niter / 2 > 0 && (st = launch_tma(h, h->tc, niter / 2, launches))) return st;
-    if (niter & 1) st = launch_tma(h, h->tail, 1, launches);
-    return st;
+    const bool one = h->dataflow && h->tc.sweeps == 2 && h->tail.ok;
+    return launch_tma(h, one ? h->tail : h->tc, niter, launches);
 }
 
 int persistent(cfm_jacobi *h, int niter, int *launches) {
@@ -1173,7 +1190,7 @@ int cfm_jacobi_create(const cfm_jacobi_params *p, cfm_jacobi **out) {
     h->own_stream = true;
     if ((st = choose_launch(h))) return fail(st);
     if (h->p.impl == CFM_JACOBI_PERSISTENT || h->p.impl == CFM_JACOBI_RESIDENT)
-        if ((st = setup_tma(h, default_tma_variant()))) return fail(st);
+        if ((st = setup_tma(h, default_tma_variant(h)))) return fail(st);
     if (h->j2.fn &&
         (e = cudaMalloc(&h->flags, sizeof(unsigned int) * h->num_sms)) != cudaSuccess) {
         set_error("exchange counters: %s", cudaGetErrorString(e));
@@ -1366,7 +1383,8 @@ int cfm_jacobi_autotune(cfm_jacobi *h, int sweeps, int *best_variant, double *be
     CFM_ARG_CHECK(sweeps >= 1, "sweeps must be >= 1");
     if (best_variant) *best_variant = -1;
     if (best_glups) *best_glups = 0.0;
-    if (!h->tma) return CFM_OK;  // only the TMA pipeline has shapes to choose from
+    // only 3D rows of 16-byte multiples have shapes to choose from
+    if (!h->tma || ((size_t)h->p.nx * h->esize) % 16 != 0) return CFM_OK;
     const size_t bytes = h->elems * h->esize;
     void *saved = nullptr;
     CFM_CUDA_TRY(cudaMalloc(&saved, bytes));
@@ -1409,7 +1427,7 @@ int cfm_jacobi_autotune(cfm_jacobi *h, int sweeps, int *best_variant, double *be
         }
     }
     const int st2 =
-        (best >= 0) ? setup_tma(h, best, best_zc) : setup_tma(h, default_tma_variant());
+        (best >= 0) ? setup_tma(h, best, best_zc) : setup_tma(h, default_tma_variant(h));
     const int st3 = restore();
     cudaFree(saved);
     CFM_CUDA_TRY(e);

@@ -30,3 +30,18 @@ def test_2d_several_sweeps_per_pass(shape, niter, prec, mirror):
         j.run(niter)
         want = (oracle.jacobi2d_mirror if mirror else oracle.jacobi2d)(a, niter)
         np.testing.assert_array_equal(j.download(), want)
+
+
+# Rows and columns at the tile edges (rows of a multiple of 16 bytes or not), z chunks that
+# end beside the periodic planes, odd and even counts.
+@pytest.mark.parametrize("py", [0, 1])
+@pytest.mark.parametrize("prec", [cfm.FP64, cfm.FP32])
+@pytest.mark.parametrize("shape,niter", [((9, 38, 64), 4), ((40, 39, 63), 5), ((12, 75, 65), 6),
+                                         ((70, 40, 127), 3), ((33, 90, 129), 7), ((6, 5, 250), 8)])
+def test_3d_two_sweeps_per_pass(shape, niter, prec, py):
+    a = rand_grid(shape, prec, 32)
+    nz, ny, nx = shape
+    with cfm.Jacobi(3, nx, ny, nz, prec, py, cfm.JACOBI_PERSISTENT) as j:
+        j.upload(a)
+        j.run(niter)
+        np.testing.assert_array_equal(j.download(), oracle.jacobi3d(a, niter, py))
