@@ -44,6 +44,12 @@ struct cfm_csr {
     int *col = nullptr;
     double *val = nullptr;
     float *val32 = nullptr;
+    // row classes (ClassOp): 0 none, 1 by column offsets, 2 by offsets and values
+    int classes = 0, L = 0;
+    unsigned char *cls = nullptr;
+    int *len = nullptr, *off = nullptr;
+    double *tval = nullptr;
+    float *tval32 = nullptr;
 };
 
 struct cfm_stencil {
@@ -74,6 +80,104 @@ struct cfm_cg {
 namespace {
 
 CsrOp csr_op(const cfm_csr *A) { return CsrOp{A->rowptr, A->col, A->val, A->val32}; }
+
+template <bool VALS>
+ClassOp<VALS> class_op(const cfm_csr *A) {
+    return ClassOp<VALS>{A->rowptr, A->val, A->val32, A->cls, A->len, A->off, A->tval, A->tval32, A->L};
+}
+
+// Groups the rows of a 0-based CSR matrix into classes of equal column offsets
+// (and values, when val is given): cls[i] per row and one representative row per
+// class.  False as soon as there are more than CLS_MAX classes or a row is longer than
+// CLS_MAXLEN.  A row is compared with its predecessor's class first, then looked up.
+bool classify_rows(int n, const int *rp, const int *col, const double *val, std::vector<unsigned char> &cls,
+                   std::vector<int> &reps) {
+    auto same = [&](int i, int j) {
+        const int m = rp[i + 1] - rp[i];
+        if (rp[j + 1] - rp[j] != m) return false;
+        const int a = rp[i], b = rp[j], d = i - j;
+        for (int k = 0; k < m; ++k)
+            if (col[a + k] - d != col[b + k]) return false;
+        return !val || m == 0 || std::memcmp(val + a, val + b, sizeof(double) * m) == 0;
+    };
+    auto hash = [&](int i) {
+        unsigned long long h = (unsigned long long)(rp[i + 1] - rp[i]) + 1;
+        auto mix = [&](unsigned long long v) { h = (h ^ v) * 0x9E3779B97F4A7C15ull, h ^= h >> 29; };
+        for (int k = rp[i]; k < rp[i + 1]; ++k) {
+            mix((unsigned)(col[k] - i));
+            if (val) {
+                unsigned long long b;
+                std::memcpy(&b, val + k, sizeof(b));
+                mix(b);
+            }
+        }
+        return h;
+    };
+    constexpr int SLOTS = 4 * CLS_MAX;
+    std::vector<int> table(SLOTS, -1);
+    cls.assign(n, 0);
+    reps.clear();
+    int last = -1;
+    for (int i = 0; i < n; ++i) {
+        if (last >= 0 && same(i, reps[last])) {
+            cls[i] = (unsigned char)last;
+            continue;
+        }
+        if (rp[i + 1] - rp[i] > CLS_MAXLEN) return false;
+        int s = (int)(hash(i) % SLOTS);
+        while (table[s] >= 0 && !same(i, reps[table[s]])) s = (s + 1) % SLOTS;
+        if (table[s] < 0) {
+            if ((int)reps.size() == CLS_MAX) return false;
+            table[s] = (int)reps.size();
+            reps.push_back(i);
+        }
+        last = table[s];
+        cls[i] = (unsigned char)last;
+    }
+    return true;
+}
+
+// Finds the matrix's row classes and uploads their tables (A->classes stays 0 when
+// there are too many).
+cudaError_t build_classes(cfm_csr *A, const int *rp, const int *col, const double *val) {
+    std::vector<unsigned char> cls;
+    std::vector<int> reps;
+    int kind = 0;
+    if (classify_rows(A->n, rp, col, val, cls, reps))
+        kind = 2;
+    else if (classify_rows(A->n, rp, col, nullptr, cls, reps))
+        kind = 1;
+    if (!kind) return cudaSuccess;
+    int L = 4;
+    for (int r : reps) L = std::max(L, (rp[r + 1] - rp[r] + 3) / 4 * 4);
+    const size_t C = reps.size(), N = C * L;
+    std::vector<int> len(C), off(N, 0);
+    std::vector<double> tv(N, 0.0);
+    std::vector<float> tv32(N, 0.f);
+    for (size_t c = 0; c < C; ++c) {
+        const int r = reps[c], b = rp[r];
+        len[c] = rp[r + 1] - b;
+        for (int k = 0; k < len[c]; ++k) {
+            off[c * L + k] = col[b + k] - r;
+            tv[c * L + k] = val[b + k];
+            tv32[c * L + k] = (float)val[b + k];
+        }
+    }
+    cudaError_t e;
+    if ((e = cudaMalloc(&A->cls, A->n)) != cudaSuccess || (e = cudaMalloc(&A->len, sizeof(int) * C)) != cudaSuccess ||
+        (e = cudaMalloc(&A->off, sizeof(int) * N)) != cudaSuccess ||
+        (e = cudaMalloc(&A->tval, sizeof(double) * N)) != cudaSuccess ||
+        (e = cudaMalloc(&A->tval32, sizeof(float) * N)) != cudaSuccess ||
+        (e = cudaMemcpy(A->cls, cls.data(), A->n, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemcpy(A->len, len.data(), sizeof(int) * C, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemcpy(A->off, off.data(), sizeof(int) * N, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemcpy(A->tval, tv.data(), sizeof(double) * N, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemcpy(A->tval32, tv32.data(), sizeof(float) * N, cudaMemcpyHostToDevice)) != cudaSuccess)
+        return e;
+    A->classes = kind;
+    A->L = L;
+    return cudaSuccess;
+}
 
 template <int D>
 StencilOp<D> stencil_op(const cfm_stencil *S) {
@@ -315,6 +419,11 @@ int solve_impl(cfm_cg *h, const double *b_dev, double *x_dev, cfm_stats *st, dou
     switch (h->kind) {
         case 2: return solve_t(h, stencil_op<2>(h->S), b_dev, x_dev, st, h2d, d2h, b_host, x_host);
         case 3: return solve_t(h, stencil_op<3>(h->S), b_dev, x_dev, st, h2d, d2h, b_host, x_host);
+        default: break;
+    }
+    switch (h->A->classes) {
+        case 1: return solve_t(h, class_op<false>(h->A), b_dev, x_dev, st, h2d, d2h, b_host, x_host);
+        case 2: return solve_t(h, class_op<true>(h->A), b_dev, x_dev, st, h2d, d2h, b_host, x_host);
         default: return solve_t(h, csr_op(h->A), b_dev, x_dev, st, h2d, d2h, b_host, x_host);
     }
 }
@@ -352,7 +461,11 @@ int create_common(cfm_cg *h, const cfm_cg_params *p) {
     switch (h->kind) {
         case 2: st = occupancy<StencilOp<2>>(p->impl, &per_sm); break;
         case 3: st = occupancy<StencilOp<3>>(p->impl, &per_sm); break;
-        default: st = occupancy<CsrOp>(p->impl, &per_sm); break;
+        default:
+            st = h->A->classes == 1   ? occupancy<ClassOp<false>>(p->impl, &per_sm)
+                 : h->A->classes == 2 ? occupancy<ClassOp<true>>(p->impl, &per_sm)
+                                      : occupancy<CsrOp>(p->impl, &per_sm);
+            break;
     }
     if (st) return st;
     if (per_sm < 1) {
@@ -484,6 +597,11 @@ int cfm_csr_create(int n, long long nnz, const int *rowptr, const int *col, cons
             return CFM_CUDA_ERROR;
         }
     }
+    if ((e = build_classes(A, rp.data(), cc.data(), val)) != cudaSuccess) {
+        set_error("csr row classes failed: %s", cudaGetErrorString(e));
+        cfm_csr_destroy(A);
+        return e == cudaErrorMemoryAllocation ? CFM_OUT_OF_MEMORY : CFM_CUDA_ERROR;
+    }
     *out = A;
     return CFM_OK;
 }
@@ -494,6 +612,11 @@ void cfm_csr_destroy(cfm_csr *A) {
     cudaFree(A->col);
     cudaFree(A->val);
     cudaFree(A->val32);
+    cudaFree(A->cls);
+    cudaFree(A->len);
+    cudaFree(A->off);
+    cudaFree(A->tval);
+    cudaFree(A->tval32);
     delete A;
 }
 

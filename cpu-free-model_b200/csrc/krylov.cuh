@@ -2,6 +2,7 @@
 //
 // Operators (one row per thread, tiles of CG_TILE consecutive rows):
 //   CsrOp        CSR SpMV, row order, one fma per nonzero (CG/src/common.cu:150-168)
+//   ClassOp      the same sums for matrices whose rows fall into few classes
 //   StencilOp<D> matrix-free cell-centred -div(k grad u), 5-point (D = 2) or
 //                7-point (D = 3): t = d_i u_i, then one fma(-w, u_nb, t) per
 //                neighbour in the order x-1, x+1, y-1, y+1, z-1, z+1
@@ -49,20 +50,39 @@ __device__ __forceinline__ double warp_xor_sum(double v) {
     return v;
 }
 
-// Tree sum over the 1024 threads of the block; every thread gets the result.
-__device__ __forceinline__ double block_sum(double v, double *sm /* 33 doubles */) {
+// Tree sum over the 1024 threads of the block; every thread gets the result (each
+// warp adds the 32 warp sums for itself, which costs no second hand-over).
+__device__ __forceinline__ double block_sum(double v, double *sm /* 32 doubles */) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     v = warp_xor_sum(v);
     if (lane == 0) sm[warp] = v;
     __syncthreads();
-    if (warp == 0) {
-        double w = warp_xor_sum(sm[lane]);
-        if (lane == 0) sm[32] = w;
-    }
-    __syncthreads();
-    const double out = sm[32];
+    const double out = warp_xor_sum(sm[lane]);
     __syncthreads();
     return out;
+}
+
+// One or two sums of tile partials in the fixed order (thread t adds part[t],
+// part[t+1024], ..., then the tree of block_sum) behind one block barrier: every warp
+// adds the 32 warp sums for itself.  sm: N x 32 doubles that no thread still reads.
+template <int N>
+__device__ __forceinline__ void partial_sums(const double *p, const double *p2, int ntiles, double *sm, double *out,
+                                             double *out2) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v = 0.0, v2 = 0.0;
+    for (int i = threadIdx.x; i < ntiles; i += CG_TILE) {
+        v = __dadd_rn(v, p[i]);
+        if (N > 1) v2 = __dadd_rn(v2, p2[i]);
+    }
+    v = warp_xor_sum(v);
+    if (N > 1) v2 = warp_xor_sum(v2);
+    if (lane == 0) {
+        sm[warp] = v;
+        if (N > 1) sm[32 + warp] = v2;
+    }
+    __syncthreads();
+    *out = warp_xor_sum(sm[lane]);
+    if (N > 1) *out2 = warp_xor_sum(sm[32 + lane]);
 }
 
 // Sum of tile partials in the fixed order: thread t adds part[t], part[t+1024], ...
@@ -153,6 +173,7 @@ struct Vals32 {
 // faster (20.1-20.9 against 19.9-20.2 ms), so those keep one entry per step.
 constexpr int CSR_Q = 4;
 struct CsrOp {
+    static constexpr bool ROW_FIRST = false;  // phase_pipe_step (its registers would spill)
     const int *rowptr, *col;
     const double *val;
     const float *val32;
@@ -223,15 +244,17 @@ struct CsrOp {
                                            double &y1, double &y2) const {
         apply2_t(val, x, i, v1, i2, v2, y1, y2);
     }
+    // What a row's loads begin with, for a caller that has time to load it ahead.
+    __device__ __forceinline__ int key(int i) const { return rowptr[i]; }
     // FP32 apply for the rows of a tile group (0 for an absent row), their
-    // entries interleaved.
+    // entries interleaved; key: key() of the rows.
     template <int U>
-    __device__ __forceinline__ Vals32<U> applyN32(const float *x, const TileGroup<U> &g) const {
+    __device__ __forceinline__ Vals32<U> applyN32(const float *x, const TileGroup<U> &g, const int (&key)[U]) const {
         int j[U], e[U];
         Vals32<U> y;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            j[u] = g.ok[u] ? rowptr[g.row[u]] : 0;
+            j[u] = g.ok[u] ? key[u] : 0;
             e[u] = g.ok[u] ? rowptr[g.row[u] + 1] : 0;
             y.v[u] = 0.f;
         }
@@ -257,13 +280,132 @@ struct CsrOp {
     }
 };
 
+// CSR matrix whose rows fall into at most 256 classes (cfm_csr_create finds
+// them): rows of a class have the same column offsets col - i and, with VALS, the
+// same values bit for bit (a constant-coefficient grid operator has one class per
+// kind of boundary).  A row then costs one byte and a table entry that stays in L1
+// instead of its column indices (and values) from L2 or HBM, and its gathers wait
+// for that byte instead of rowptr and col in turn.  Entries are taken in row order,
+// so the sums are CsrOp's bit for bit.  Table rows are L entries (a multiple of 4).
+constexpr int CLS_MAX = 256, CLS_MAXLEN = 32;
+template <bool VALS>
+struct ClassOp {
+    static constexpr bool ROW_FIRST = true;
+    const int *rowptr;
+    const double *val;
+    const float *val32;
+    const unsigned char *cls;
+    const int *len, *off;  // per class: entries, offsets
+    const double *tval;    // VALS: per class values
+    const float *tval32;
+    int L;
+    __device__ __forceinline__ static double fma_rn(double u, double w, double c) { return __fma_rn(u, w, c); }
+    __device__ __forceinline__ static float fma_rn(float u, float w, float c) { return __fmaf_rn(u, w, c); }
+    // 16 bytes of a value row, and as many offsets
+    __device__ __forceinline__ static void load(const double *p, double (&v)[2]) {
+        const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
+        v[0] = a.x, v[1] = a.y;
+    }
+    __device__ __forceinline__ static void load(const float *p, float (&v)[4]) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    }
+    __device__ __forceinline__ static void load(const int *p, int (&v)[2]) {
+        const int2 a = __ldg(reinterpret_cast<const int2 *>(p));
+        v[0] = a.x, v[1] = a.y;
+    }
+    __device__ __forceinline__ static void load(const int *p, int (&v)[4]) {
+        const int4 a = __ldg(reinterpret_cast<const int4 *>(p));
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    }
+    // Row i's class, for a caller that has time to load it ahead of the row.
+    __device__ __forceinline__ int key(int i) const { return cls[i]; }
+    // The rows of a group (those with ok; c: their classes), C entries of each at a time,
+    // their gathers (and, without VALS, values) in flight together; 0 for an absent row.
+    // With VALS the values come from the table (L1) only as they are used, which leaves
+    // the registers to the gathers: a 7-point row takes one step in FP32, two in FP64.
+    template <int U, class T>
+    __device__ __forceinline__ void rows(const T *v, const T *tv, const T *x, const int (&row)[U],
+                                         const bool (&ok)[U], const int (&c)[U], T (&y)[U]) const {
+        constexpr int Q = 16 / sizeof(T), C = Q;
+        int m[U], at[U], src[U], most = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            m[u] = ok[u] ? __ldg(len + c[u]) : 0;
+            at[u] = c[u] * L;
+            src[u] = !VALS && ok[u] ? rowptr[row[u]] : 0;
+            most = max(most, m[u]);
+            y[u] = T(0);
+        }
+#pragma unroll 1
+        for (int k = 0; k < most; k += C) {
+            T w[U][VALS ? 1 : C], g[U][C];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int h = 0; h < C; h += Q) {
+                    if (k + h >= m[u]) continue;
+                    int o[Q];
+                    load(off + at[u] + k + h, o);
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) {
+                        const bool in = k + h + q < m[u];
+                        if (!VALS) w[u][VALS ? 0 : h + q] = in ? v[src[u] + k + h + q] : T(0);
+                        g[u][h + q] = in ? x[row[u] + o[q]] : T(0);
+                    }
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int h = 0; h < C; h += Q) {
+                    if (k + h >= m[u]) continue;
+                    T t[Q];
+                    if (VALS) load(tv + at[u] + k + h, t);
+#pragma unroll
+                    for (int q = 0; q < Q; ++q)
+                        if (k + h + q < m[u]) y[u] = fma_rn(VALS ? t[q] : w[u][VALS ? 0 : h + q], g[u][h + q], y[u]);
+                }
+        }
+    }
+    __device__ __forceinline__ double apply(const double *x, int i) const {
+        const int row[1] = {i}, c[1] = {cls[i]};
+        const bool ok[1] = {true};
+        double y[1];
+        rows<1>(val, tval, x, row, ok, c, y);
+        return y[0];
+    }
+    __device__ __forceinline__ void apply2(const double *x, int i, bool v1, int i2, bool v2, double &y1,
+                                           double &y2) const {
+        const int row[2] = {i, i2}, c[2] = {v1 ? cls[i] : 0, v2 ? cls[i2] : 0};
+        const bool ok[2] = {v1, v2};
+        double y[2];
+        rows<2>(val, tval, x, row, ok, c, y);
+        y1 = y[0];
+        y2 = y[1];
+    }
+    template <int U>
+    __device__ __forceinline__ Vals32<U> applyN32(const float *x, const TileGroup<U> &g, const int (&key)[U]) const {
+        Vals32<U> y;
+        rows<U>(val32, tval32, x, g.row, g.ok, key, y.v);
+        return y;
+    }
+    // A x0 with x0 = 0, summed like apply (always +0)
+    __device__ __forceinline__ double apply_zero(int i) const {
+        const int c = cls[i], m = __ldg(len + c);
+        double acc = 0.0;
+        for (int k = 0; k < m; ++k) acc = __fma_rn(VALS ? __ldg(tval + c * L + k) : val[rowptr[i] + k], 0.0, acc);
+        return acc;
+    }
+};
+
 template <int D>
 struct StencilOp {
+    static constexpr bool ROW_FIRST = true;
     int nx, ny, nz;
     const double *we, *wn, *wt, *dg;
     const float *we32, *wn32, *wt32, *dg32;
     __device__ __forceinline__ double apply(const double *x, int i) const {
-        const int ix = i % nx, q = i / nx, iy = q % ny;
+        const int q = i / nx, ix = i - q * nx, iy = D == 3 ? q % ny : q;
         double t = __dmul_rn(dg[i], x[i]);
         if (ix > 0) t = __fma_rn(-we[i - 1], x[i - 1], t);
         if (ix < nx - 1) t = __fma_rn(-we[i], x[i + 1], t);
@@ -277,7 +419,7 @@ struct StencilOp {
         return t;
     }
     __device__ __forceinline__ float apply32(const float *x, int i) const {
-        const int ix = i % nx, q = i / nx, iy = q % ny;
+        const int q = i / nx, ix = i - q * nx, iy = D == 3 ? q % ny : q;
         float t = __fmul_rn(dg32[i], x[i]);
         if (ix > 0) t = __fmaf_rn(-we32[i - 1], x[i - 1], t);
         if (ix < nx - 1) t = __fmaf_rn(-we32[i], x[i + 1], t);
@@ -296,8 +438,9 @@ struct StencilOp {
         y1 = v1 ? apply(x, i) : 0.0;
         y2 = v2 ? apply(x, i2) : 0.0;
     }
+    __device__ __forceinline__ int key(int) const { return 0; }
     template <int U>
-    __device__ __forceinline__ Vals32<U> applyN32(const float *x, const TileGroup<U> &g) const {
+    __device__ __forceinline__ Vals32<U> applyN32(const float *x, const TileGroup<U> &g, const int (&)[U]) const {
         Vals32<U> y;
 #pragma unroll
         for (int u = 0; u < U; ++u) y.v[u] = g.ok[u] ? apply32(x, g.row[u]) : 0.f;
@@ -344,6 +487,32 @@ template <class Op>
 __device__ __forceinline__ double *slot(const KArgs<Op> &a, int s) {
     return a.part + (size_t)s * a.ntiles;
 }
+
+// A persistent solver's barriers and grid-wide sums: a sum is a barrier, after which
+// every block adds the tile partials of a slot (or two) in sum_partials' order.  Each
+// returns false once a wait ran out.
+template <class Op>
+struct CgGrid {
+    const KArgs<Op> &a;
+    double *red;  // 4 x 32 doubles of shared memory, used by turns
+    int site = 0, par = 0;
+    __device__ __forceinline__ CgGrid(const KArgs<Op> &args, double *r) : a(args), red(r) {}
+    __device__ __forceinline__ bool barrier() { return grid_barrier(a.bar, gridDim.x, site++); }
+    __device__ __forceinline__ bool sum(int s, double *out) {
+        if (!barrier()) return false;
+        sums<1>(slot(a, s), nullptr, out, nullptr);
+        return true;
+    }
+    __device__ __forceinline__ bool sum2(int s, double *out, int s2, double *out2) {
+        if (!barrier()) return false;
+        sums<2>(slot(a, s), slot(a, s2), out, out2);
+        return true;
+    }
+    template <int N>
+    __device__ __forceinline__ void sums(const double *p, const double *p2, double *out, double *out2) {
+        partial_sums<N>(p, p2, a.ntiles, red + 64 * (par ^= 1), out, out2);
+    }
+};
 
 // -------------------------------------------------------- standard phases
 template <class Op>
@@ -492,12 +661,12 @@ __device__ __forceinline__ void write_result(CgResult *res, long long k, int sta
 // otherwise); tol <= 0 runs exactly maxiter iterations (reference -niter).
 template <class Op>
 __global__ void __launch_bounds__(CG_TILE, 1) cg_std_kernel(KArgs<Op> a) {
-    __shared__ double sm[TS_SMEM];
-    int site = 0;
+    __shared__ double sm[TS_SMEM], red[128];
+    CgGrid<Op> grid(a, red);
     phase_init(a, sm);
-    if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-    double gamma0 = sum_partials(slot(a, SL_G0), a.ntiles, sm);
-    const double bnorm = sqrt(sum_partials(slot(a, SL_B), a.ntiles, sm));
+    double gamma0, bb;
+    if (!grid.sum2(SL_G0, &gamma0, SL_B, &bb)) return;
+    const double bnorm = sqrt(bb);
     const bool use_tol = a.tol > 0.0;
     const double target = a.tol * bnorm;
     int status = use_tol ? CFM_NOT_CONVERGED : CFM_OK;
@@ -506,23 +675,23 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_std_kernel(KArgs<Op> a) {
     if (use_tol && sqrt(gamma0) <= target) status = CFM_OK;
     while (k < a.maxiter && !(use_tol && status == CFM_OK)) {
         phase_spmv_dot(a, sm);
-        if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-        const double delta = sum_partials(slot(a, SL_D0), a.ntiles, sm);
+        double delta;
+        if (!grid.sum(SL_D0, &delta)) return;
         const double alpha = gamma0 / delta;
         if (use_tol && !(delta > 0.0 && isfinite(alpha))) {
             status = CFM_BREAKDOWN;
             break;
         }
         phase_update(a, alpha, sm);
-        if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-        const double gamma1 = sum_partials(slot(a, SL_G0), a.ntiles, sm);
+        double gamma1;
+        if (!grid.sum(SL_G0, &gamma1)) return;
         ++k;
         if (a.snap && k % a.snap_every == 0 && k / a.snap_every <= a.snap_max)
             phase_snap(a, (int)(k / a.snap_every) - 1);  // x is stable until the next update
         if (use_tol && sqrt(gamma1) <= target) {
             phase_true_residual(a, sm);
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-            const double tt = sum_partials(slot(a, SL_TT), a.ntiles, sm);
+            double tt;
+            if (!grid.sum(SL_TT, &tt)) return;
             if (sqrt(tt) <= target) {
                 status = CFM_OK;
                 gamma0 = gamma1;
@@ -531,7 +700,7 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_std_kernel(KArgs<Op> a) {
             phase_restart(a);
             ++restarts;
             gamma0 = tt;
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
+            if (!grid.barrier()) return;
             continue;
         }
         const double beta = gamma1 / gamma0;
@@ -540,7 +709,7 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_std_kernel(KArgs<Op> a) {
             break;
         }
         phase_p(a, beta);
-        if (!grid_barrier(a.bar, gridDim.x, site++)) return;
+        if (!grid.barrier()) return;
         gamma0 = gamma1;
     }
     write_result(a.res, k, status, restarts, gamma0, bnorm);
@@ -602,13 +771,17 @@ __device__ void phase_pipe_step(const KArgs<Op> &a, const double *w, double *wn,
         CFM_ROW(a);
         double g = 0.0, d = 0.0;
         if (i < a.n) {
-            const double q = a.op.apply(w, i);
-            const double wi = w[i];
-            const double zi = __fma_rn(beta, a.z[i], q);
-            const double si = __fma_rn(beta, a.s[i], wi);
-            const double pi = __fma_rn(beta, a.p[i], a.r[i]);
-            a.x[i] = __fma_rn(alpha, pi, a.x[i]);
-            const double ri = __fma_rn(-alpha, si, a.r[i]);
+            // ROW_FIRST: the row's own entries are in flight while the operator's chain of
+            // loads runs
+            double wi, z0, s0, p0, r0, x0, q;
+            if (!Op::ROW_FIRST) q = a.op.apply(w, i);
+            wi = w[i], z0 = a.z[i], s0 = a.s[i], p0 = a.p[i], r0 = a.r[i], x0 = a.x[i];
+            if (Op::ROW_FIRST) q = a.op.apply(w, i);
+            const double zi = __fma_rn(beta, z0, q);
+            const double si = __fma_rn(beta, s0, wi);
+            const double pi = __fma_rn(beta, p0, r0);
+            a.x[i] = __fma_rn(alpha, pi, x0);
+            const double ri = __fma_rn(-alpha, si, r0);
             const double wni = __fma_rn(-alpha, zi, wi);
             a.z[i] = zi;
             a.s[i] = si;
@@ -672,13 +845,13 @@ constexpr long long PIPE_REPLACE = 50;
 // extra barriers, four operator applications); the scalar recurrence goes on.
 template <class Op>
 __global__ void __launch_bounds__(CG_TILE, 1) cg_pipe_kernel(KArgs<Op> a) {
-    __shared__ double sm[TS_SMEM];
-    int site = 0;
+    __shared__ double sm[TS_SMEM], red[128];
+    CgGrid<Op> grid(a, red);
     phase_pipe_init(a, sm);
-    if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-    const double bnorm = sqrt(sum_partials(slot(a, SL_B), a.ntiles, sm));
+    double bb;
+    if (!grid.sum(SL_B, &bb)) return;
+    const double bnorm = sqrt(bb);
     phase_pipe_start(a, a.t, a.w0, 0, sm);
-    if (!grid_barrier(a.bar, gridDim.x, site++)) return;
     const bool use_tol = a.tol > 0.0;
     const double target = a.tol * bnorm;
     int status = use_tol ? CFM_NOT_CONVERGED : CFM_OK;
@@ -687,18 +860,17 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_pipe_kernel(KArgs<Op> a) {
     double rr = 0.0, rr_prev = 0.0, alpha = 0.0;
     while (true) {
         double *w = cur ? a.w1 : a.w0;
-        rr = sum_partials(slot(a, cur ? SL_G1 : SL_G0), a.ntiles, sm);
-        const double wr = sum_partials(slot(a, cur ? SL_D1 : SL_D0), a.ntiles, sm);
+        double wr;
+        if (!grid.sum2(cur ? SL_G1 : SL_G0, &rr, cur ? SL_D1 : SL_D0, &wr)) return;
         if (use_tol && sqrt(rr) <= target) {
             phase_true_residual(a, sm);
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-            const double tt = sum_partials(slot(a, SL_TT), a.ntiles, sm);
+            double tt;
+            if (!grid.sum(SL_TT, &tt)) return;
             if (sqrt(tt) <= target) {
                 status = CFM_OK;
                 break;
             }
             phase_pipe_start(a, a.t, w, cur, sm);  // restart from the true residual
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
             ++restarts;
             kk = 0;
             replaced = k;  // a restart needs no replacement at this count
@@ -707,9 +879,8 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_pipe_kernel(KArgs<Op> a) {
         if (k >= a.maxiter) break;
         if (use_tol && k > 0 && k % PIPE_REPLACE == 0 && replaced != k) {
             phase_replace_a(a);
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
+            if (!grid.barrier()) return;
             phase_replace_b(a, w, cur, sm);
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
             replaced = k;
             ++restarts;
             continue;
@@ -727,7 +898,6 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_pipe_kernel(KArgs<Op> a) {
             break;
         }
         phase_pipe_step(a, w, cur ? a.w0 : a.w1, alpha, beta, cur ^ 1, sm);
-        if (!grid_barrier(a.bar, gridDim.x, site++)) return;
         rr_prev = rr;
         cur ^= 1;
         ++k;
@@ -777,22 +947,36 @@ __device__ void phase_inner_start(const KArgs<Op> &a, double scale, double *sm) 
     ts.flush();
 }
 
+// The FP32 passes load a group's own values while the group before it is worked on:
+// a block has few groups (seven at 128^3), and each otherwise waits out a round trip.
 template <class Op>
 __device__ void phase_inner_spmv(const KArgs<Op> &a, double *sm) {
     constexpr int U = INNER_U;
     TileSums<1> ts(sm, gridDim.x, slot(a, SL_D0));
+    float p[U];
+    int key[U];
+    auto load = [&](const TileGroup<U> &g, float (&pv)[U], int (&kv)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            pv[u] = g.ok[u] ? a.p32[g.row[u]] : 0.f;
+            kv[u] = g.ok[u] ? a.op.key(g.row[u]) : 0;
+        }
+    };
+    load(TileGroup<U>(a.ntiles, a.n, blockIdx.x), p, key);
     CFM_TILE_GROUPS(a, U) {
         const TileGroup<U> g(a.ntiles, a.n, tile);
-        float p[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) p[u] = g.ok[u] ? a.p32[g.row[u]] : 0.f;
-        const Vals32<U> y = a.op.template applyN32<U>(a.p32, g);
+        float pn[U];
+        int kn[U];
+        load(TileGroup<U>(a.ntiles, a.n, tile + U * (int)gridDim.x), pn, kn);
+        const Vals32<U> y = a.op.template applyN32<U>(a.p32, g, key);
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (g.ok[u]) a.s32[g.row[u]] = y.v[u];
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (g.has[u]) ts.add(g.tile[u], g.ok[u] ? xprod(p[u], y.v[u]) : 0.0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) p[u] = pn[u], key[u] = kn[u];
     }
     ts.flush();
 }
@@ -801,37 +985,44 @@ template <class Op>
 __device__ void phase_inner_update(const KArgs<Op> &a, float af, double *sm) {
     constexpr int U = INNER_U;
     TileSums<1> ts(sm, gridDim.x, slot(a, SL_G0));
-    CFM_TILE_GROUPS(a, U) {
-        const TileGroup<U> g(a.ntiles, a.n, tile);
-        float d[U], p[U], r[U], sv[U];
+    struct Own {
+        float d[U], p[U], r[U], s[U];
+    } cur, nxt;
+    auto load = [&](const TileGroup<U> &g, Own &v) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            d[u] = p[u] = r[u] = sv[u] = 0.f;
+            v.d[u] = v.p[u] = v.r[u] = v.s[u] = 0.f;
             if (g.ok[u]) {
-                d[u] = a.d32[g.row[u]];
-                p[u] = a.p32[g.row[u]];
-                r[u] = a.r32[g.row[u]];
-                sv[u] = a.s32[g.row[u]];
+                v.d[u] = a.d32[g.row[u]];
+                v.p[u] = a.p32[g.row[u]];
+                v.r[u] = a.r32[g.row[u]];
+                v.s[u] = a.s32[g.row[u]];
             }
         }
+    };
+    load(TileGroup<U>(a.ntiles, a.n, blockIdx.x), cur);
+    CFM_TILE_GROUPS(a, U) {
+        const TileGroup<U> g(a.ntiles, a.n, tile);
+        load(TileGroup<U>(a.ntiles, a.n, tile + U * (int)gridDim.x), nxt);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             double q = 0.0;
             if (g.ok[u]) {
-                a.d32[g.row[u]] = __fmaf_rn(af, p[u], d[u]);
-                const float ri = __fmaf_rn(-af, sv[u], r[u]);
+                a.d32[g.row[u]] = __fmaf_rn(af, cur.p[u], cur.d[u]);
+                const float ri = __fmaf_rn(-af, cur.s[u], cur.r[u]);
                 a.r32[g.row[u]] = ri;
                 q = xprod(ri, ri);
             }
             if (g.has[u]) ts.add(g.tile[u], q);
         }
+        cur = nxt;
     }
     ts.flush();
 }
 
 template <class Op>
 __device__ void phase_inner_p(const KArgs<Op> &a, float bf) {
-    constexpr int U = INNER_U;
+    constexpr int U = 2 * INNER_U;
     CFM_TILE_GROUPS(a, U) {
         const TileGroup<U> g(a.ntiles, a.n, tile);
         float p[U], r[U];
@@ -896,13 +1087,13 @@ __device__ void phase_replace32(const KArgs<Op> &a, double scale, double *sm) {
 // residual |b - A x| <= tol |b|; maxiter caps the FP32 steps.
 template <class Op>
 __global__ void __launch_bounds__(CG_TILE, 1) cg_mixed_kernel(KArgs<Op> a) {
-    __shared__ double sm[TS_SMEM];
-    int site = 0;
+    __shared__ double sm[TS_SMEM], red[128];
+    CgGrid<Op> grid(a, red);
     phase_mixed_init(a, sm);
-    if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-    const double bnorm = sqrt(sum_partials(slot(a, SL_B), a.ntiles, sm));
+    double bb, tt;
+    if (!grid.sum2(SL_B, &bb, SL_TT, &tt)) return;
+    const double bnorm = sqrt(bb);
     const double target = a.tol * bnorm;
-    double tt = sum_partials(slot(a, SL_TT), a.ntiles, sm);
     int status = CFM_NOT_CONVERGED, updates = 0;
     long long k = 0;
     if (sqrt(tt) <= target || bnorm == 0.0) {
@@ -912,31 +1103,30 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_mixed_kernel(KArgs<Op> a) {
     const double scale = 1.0 / bnorm, tol2 = a.tol * a.tol;
     const double delta2 = a.inner_tol * a.inner_tol;
     phase_inner_start(a, scale, sm);
-    if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-    double g0 = sum_partials(slot(a, SL_G0), a.ntiles, sm), gmax = g0;
+    double g0;
+    if (!grid.sum(SL_G0, &g0)) return;
+    double gmax = g0;
     int since = 0;
     while (k < a.maxiter) {
         phase_inner_spmv(a, sm);
-        if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-        const double delta = sum_partials(slot(a, SL_D0), a.ntiles, sm);
+        double delta;
+        if (!grid.sum(SL_D0, &delta)) return;
         const double alpha = g0 / delta;
         if (!(delta > 0.0 && isfinite(alpha))) {
             status = CFM_BREAKDOWN;
             break;
         }
         phase_inner_update(a, __double2float_rn(alpha), sm);
-        if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-        double g1 = sum_partials(slot(a, SL_G0), a.ntiles, sm);
+        double g1;
+        if (!grid.sum(SL_G0, &g1)) return;
         ++k;
         ++since;
         if (g1 <= tol2 || g1 < delta2 * gmax || k >= a.maxiter ||
             (a.inner_maxiter > 0 && since >= a.inner_maxiter)) {
             phase_correct(a, bnorm);
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
+            if (!grid.barrier()) return;
             phase_replace32(a, scale, sm);
-            if (!grid_barrier(a.bar, gridDim.x, site++)) return;
-            tt = sum_partials(slot(a, SL_TT), a.ntiles, sm);
-            g1 = sum_partials(slot(a, SL_G0), a.ntiles, sm);
+            if (!grid.sum2(SL_TT, &tt, SL_G0, &g1)) return;
             ++updates;
             since = 0;
             gmax = g1;
@@ -950,7 +1140,7 @@ __global__ void __launch_bounds__(CG_TILE, 1) cg_mixed_kernel(KArgs<Op> a) {
         }
         const double beta = g1 / g0;
         phase_inner_p(a, __double2float_rn(beta));
-        if (!grid_barrier(a.bar, gridDim.x, site++)) return;
+        if (!grid.barrier()) return;
         g0 = g1;
     }
     if (since > 0) phase_correct(a, bnorm);  // a breakdown left steps in d32

@@ -45,3 +45,85 @@ def test_3d_two_sweeps_per_pass(shape, niter, prec, py):
         j.upload(a)
         j.run(niter)
         np.testing.assert_array_equal(j.download(), oracle.jacobi3d(a, niter, py))
+
+
+def grid_matrix(shape, values):
+    """5-point CSR matrix of a grid: constant values (few row classes with equal values),
+    or random symmetric ones (few classes of offsets only)."""
+    ny, nx = shape
+    rng = np.random.default_rng(34)
+    we = np.ones((ny, nx)) if values == "constant" else rng.uniform(0.5, 1.5, (ny, nx))
+    wn = np.ones((ny, nx)) if values == "constant" else rng.uniform(0.5, 1.5, (ny, nx))
+    rowptr, col, val = [0], [], []
+    for y in range(ny):
+        for x in range(nx):
+            i = y * nx + x
+            ent = [(i, 8.0)]
+            if x:
+                ent.append((i - 1, -we[y, x - 1]))
+            if x < nx - 1:
+                ent.append((i + 1, -we[y, x]))
+            if y:
+                ent.append((i - nx, -wn[y - 1, x]))
+            if y < ny - 1:
+                ent.append((i + nx, -wn[y, x]))
+            ent.sort()
+            col += [c for c, _ in ent]
+            val += [v for _, v in ent]
+            rowptr.append(len(col))
+    return np.array(rowptr, np.int32), np.array(col, np.int32), np.array(val)
+
+
+def many_offsets_matrix(n):
+    """Tridiagonal plus one symmetric far entry per row pair at growing distances: more
+    than 256 kinds of rows, so no row classes."""
+    far = {}
+    for i in range(0, n // 2):
+        j = n - 1 - i
+        if j - i > 1:
+            far[i], far[j] = j, i
+    rowptr, col, val = [0], [], []
+    for i in range(n):
+        ent = {i: 8.0}
+        if i:
+            ent[i - 1] = -1.0
+        if i < n - 1:
+            ent[i + 1] = -1.0
+        if i in far:
+            ent[far[i]] = -0.5
+        for c in sorted(ent):
+            col.append(c)
+            val.append(ent[c])
+        rowptr.append(len(col))
+    return np.array(rowptr, np.int32), np.array(col, np.int32), np.array(val)
+
+
+@pytest.mark.parametrize("base", [0, 1])
+@pytest.mark.parametrize("impl,method", [(cfm.CG_PERSISTENT, oracle.STD), (cfm.CG_DISCRETE, oracle.STD),
+                                         (cfm.CG_PERSISTENT_PIPELINED, oracle.PIPELINED),
+                                         (cfm.CG_MIXED, oracle.MIXED)])
+@pytest.mark.parametrize("kind", ["constant", "variable", "many"])
+def test_cg_row_classes(kind, impl, method, base):
+    rowptr, col, val = many_offsets_matrix(1301) if kind == "many" else grid_matrix((61, 47), kind)
+    b = cfm.uniform(35, len(rowptr) - 1)
+    xo, st_o, it_o, rs_o, _ = oracle.krylov_csr(rowptr, col, val, b, method, 2000, 1e-8)
+    A = cfm.CSR(rowptr + base, col + base, val)
+    x, st = cfm.CG(A, impl, 2000, 1e-8).solve(b)
+    assert st.status == st_o and st.iterations == it_o and st.refinements == rs_o
+    np.testing.assert_array_equal(x, xo)
+
+
+def test_cg_many_tiles_repeated():
+    """More tiles than threads in a block (the sums behind a barrier), and a handle used
+    again: the partials and flags of the first solve are still there."""
+    n = 1100 * 1024 + 5
+    rowptr, col, val = cfm.tridiag(n)
+    A = cfm.CSR(rowptr, col, val)
+    b = cfm.uniform(36, n)
+    for impl, method in ((cfm.CG_PERSISTENT, oracle.STD), (cfm.CG_PERSISTENT_PIPELINED, oracle.PIPELINED)):
+        h = cfm.CG(A, impl, 9, 0.0)
+        xo, _, it_o, _, _ = oracle.krylov_csr(rowptr, col, val, b, method, 9, 0.0)
+        for _ in range(3):
+            x, st = h.solve(b)
+            assert st.iterations == it_o
+            np.testing.assert_array_equal(x, xo)
