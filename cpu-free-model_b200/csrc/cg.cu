@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "cfm_internal.h"
+#include "cg_resident.cuh"
 #include "krylov.cuh"
 
 namespace cfm {
@@ -75,6 +76,11 @@ struct cfm_cg {
     bool own_stream = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int blocks = 0;
+    // standard CG with a small stencil system on chip (cg_std_res_kernel):
+    // kernel (nullptr: cg_std_kernel) and shape
+    const void *res_fn = nullptr;
+    int res_blocks = 0;
+    size_t res_smem = 0;
 };
 
 namespace {
@@ -317,6 +323,58 @@ int true_relres(cfm_cg *h, const KArgs<Op> &a, double bnorm, double *out) {
     return CFM_OK;
 }
 
+// cg_std_res_kernel for T tiles per block.
+template <int D>
+const void *resident_fn(int T) {
+    switch (T) {
+        case 1: return (const void *)cg_std_res_kernel<D, 1>;
+        case 2: return (const void *)cg_std_res_kernel<D, 2>;
+        case 3: return (const void *)cg_std_res_kernel<D, 3>;
+        case 4: return (const void *)cg_std_res_kernel<D, 4>;
+        default: return (const void *)cg_std_res_kernel<D, 6>;
+    }
+}
+
+// Standard CG on a stencil runs on chip when one block per SM holds the whole
+// system: the fewest tiles per block that do, up to the shared memory.
+int plan_resident(cfm_cg *h, const DeviceInfo &di) {
+    if (h->p.impl != CFM_CG_PERSISTENT || h->kind == 0) return CFM_OK;
+    for (int T : {1, 2, 3, 4, 6}) {
+        const int blocks = (h->ntiles + T - 1) / T;
+        if (blocks > di.num_sms) continue;
+        const size_t smem = sizeof(double) * (h->kind == 2 ? cgr_smem_doubles<2>(T, h->S->nx, h->S->ny)
+                                                           : cgr_smem_doubles<3>(T, h->S->nx, h->S->ny));
+        if (smem > di.smem_optin) return CFM_OK;
+        const void *fn = h->kind == 2 ? resident_fn<2>(T) : resident_fn<3>(T);
+        CFM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int per_sm = 0;
+        CFM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, CG_TILE, smem));
+        if (per_sm < 1) return CFM_OK;
+        h->res_fn = fn;
+        h->res_blocks = blocks;
+        h->res_smem = smem;
+        return CFM_OK;
+    }
+    return CFM_OK;
+}
+
+template <class Op>
+const void *solver_fn(int impl);
+
+// The handle's persistent solver for these arguments.
+template <class Op>
+int launch_solver(cfm_cg *h, KArgs<Op> &a) {
+    void *args[] = {&a};
+    if (h->res_fn) {
+        CFM_CUDA_TRY(launch_cooperative(h->res_fn, dim3(h->res_blocks), dim3(CG_TILE), args, h->res_smem,
+                                        h->stream));
+        return CFM_OK;
+    }
+    CFM_CUDA_TRY(launch_cooperative(solver_fn<Op>(h->p.impl), dim3(h->blocks), dim3(CG_TILE), args, 0,
+                                    h->stream));
+    return CFM_OK;
+}
+
 template <class Op>
 const void *solver_fn(int impl) {
     switch (impl) {
@@ -366,9 +424,7 @@ int solve_t(cfm_cg *h, const Op &op, const double *b_dev, double *x_dev, cfm_sta
         int e = run_discrete(h, a, &r, &launches);
         if (e) return e;
     } else {
-        void *args[] = {&a};
-        CFM_CUDA_TRY(launch_cooperative(solver_fn<Op>(h->p.impl), dim3(h->blocks), dim3(CG_TILE),
-                                        args, 0, h->stream));
+        if (int e = launch_solver(h, a)) return e;
         launches += 1;
     }
     if (x_host) {
@@ -473,7 +529,7 @@ int create_common(cfm_cg *h, const cfm_cg_params *p) {
         return CFM_UNSUPPORTED;
     }
     h->blocks = std::min(per_sm * di.num_sms, h->ntiles);
-    return CFM_OK;
+    return plan_resident(h, di);
 }
 
 int check_cg_params(const cfm_cg_params *p) {
@@ -514,9 +570,7 @@ int cg_stencil_snapshots(const cfm_stencil *S, const double *b_dev, double *x_de
         BarrierState bs{};
         bs.timeout_ns = barrier_timeout_ns();
         CFM_CUDA_TRY(cudaMemcpyAsync(h->bar, &bs, sizeof(bs), cudaMemcpyHostToDevice, h->stream));
-        void *args[] = {&a};
-        CFM_CUDA_TRY(launch_cooperative((const void *)cg_std_kernel<decltype(op)>, dim3(h->blocks),
-                                        dim3(CG_TILE), args, 0, h->stream));
+        if (int e = launch_solver(h, a)) return e;
         CgResult r{};
         CFM_CUDA_TRY(cudaMemcpyAsync(&bs, h->bar, sizeof(bs), cudaMemcpyDeviceToHost, h->stream));
         CFM_CUDA_TRY(cudaMemcpyAsync(&r, h->res, sizeof(r), cudaMemcpyDeviceToHost, h->stream));

@@ -47,6 +47,21 @@ def test_3d_two_sweeps_per_pass(shape, niter, prec, py):
         np.testing.assert_array_equal(j.download(), oracle.jacobi3d(a, niter, py))
 
 
+# One tile in all, one per block, two, three, four and six per block; systems whose rows all
+# have neighbours in other blocks; beyond the chip.
+@pytest.mark.parametrize("shape,maxiter", [((20, 30), 400), ((33, 31), 400), ((300, 200), 60), ((450, 500), 40),
+                                           ((600, 640), 30), ((760, 700), 30), ((930, 900), 20), ((1100, 1000), 20),
+                                           ((50, 50, 50), 60), ((80, 75, 70), 30), ((100, 100, 90), 20)])
+def test_cg_system_on_chip(shape, maxiter):
+    k, f = cfm.varcoef_problem(shape, 33)
+    dims = len(shape)
+    grid = (shape[-1], shape[-2], shape[0] if dims == 3 else 1)
+    xo, st_o, it_o, rs_o, _ = oracle.krylov_stencil(dims, grid, cfm.varcoef_coeffs(k), f, oracle.STD, maxiter, 1e-8)
+    x, st = cfm.CG(cfm.Stencil(k), cfm.CG_PERSISTENT, maxiter, 1e-8).solve(f.ravel())
+    assert st.status == st_o and st.iterations == it_o and st.refinements == rs_o
+    np.testing.assert_array_equal(x, xo)
+
+
 def grid_matrix(shape, values):
     """5-point CSR matrix of a grid: constant values (few row classes with equal values),
     or random symmetric ones (few classes of offsets only)."""
