@@ -424,6 +424,24 @@ __device__ void block_sum_multi(double *v, int nv, double *sm) {
     __syncthreads();
 }
 
+// Two tile partials (block_sum's trees) behind one block barrier, stored by one thread.
+// sm: 64 doubles.
+__device__ __forceinline__ void block_partials2(double v0, double v1, double *sm, double *d0, double *d1) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v0 = warp_xor_sum(v0);
+    v1 = warp_xor_sum(v1);
+    if (lane == 0) {
+        sm[warp] = v0;
+        sm[32 + warp] = v1;
+    }
+    __syncthreads();
+    if (warp < 2) {
+        const double v = warp_xor_sum(sm[warp * 32 + lane]);
+        if (lane == 0) *(warp ? d1 : d0) = v;
+    }
+    __syncthreads();
+}
+
 #define FP_ROW const int i = blockIdx.x * CG_TILE + threadIdx.x
 
 // x = 0, r = b; partials |b|^2, |r|^2.
@@ -499,7 +517,7 @@ __device__ __forceinline__ bool fp_inside(const FpTile &t, const FpArgs &a, int 
 // z0[l] = init(l, row, col, inside, global index, wd[l], r[l]) for every
 // region cell; the margins of this thread's cells go to mg[].
 template <class Init>
-__device__ FpTile fp_tile(const FpArgs &a, int bx, int H, unsigned char *smem, int *mg, Init init) {
+__device__ __forceinline__ FpTile fp_tile(const FpArgs &a, int bx, int H, unsigned char *smem, int *mg, Init init) {
     FpTile t;
     t.x0 = (bx % a.tx2) * FP_TILE;
     t.y0 = (bx / a.tx2) * FP_TILE;
@@ -545,7 +563,7 @@ __device__ __forceinline__ float fp_apply(const FpTile &t, const float *u, int l
 // holding the result, valid at margin m0 + sweeps.  Sweep s updates the
 // cells of margin >= m0 + s + 1 only, so it reads only cells the previous
 // sweep (or the start) wrote.
-__device__ float *fp_sweeps(const FpTile &t, const int *mg, float *cur, float *nxt, int m0, int sweeps) {
+__device__ __forceinline__ float *fp_sweeps(const FpTile &t, const int *mg, float *cur, float *nxt, int m0, int sweeps) {
     for (int s = 0; s < sweeps; ++s) {
         const int m = m0 + s + 1;
 #pragma unroll
@@ -567,15 +585,24 @@ __device__ float *fp_sweeps(const FpTile &t, const int *mg, float *cur, float *n
 // |r|^2 history, convergence / stall test]; z0 = `smooth` sweeps from zero
 // and, when the network follows (`net_next`), r1 = r - A z0, partial
 // |r1|^2, and the network input channel 0 = R(r1) (f x f means; the network
-// scales it by 1 / rms(r1) itself).
+// scales it by 1 / rms(r1) itself).  net_next & 2: R(r1) goes to the network's output
+// instead (no network: the identity stands in, and c absorbs the scale).
+// SM: the sweeps when known at compile time (the region's divisions and strides are
+// constants then; k_fp_pre<4> and k_fp_post<4> serve the default depth), else 0.
+template <int SM>
 __device__ __forceinline__ void k_fp_pre_blk(const FpArgs &a, int bx, int tick, int net_next) {
     __syncthreads();  // a previous call on this block has read its shared tile
     extern __shared__ __align__(16) unsigned char fp_smem[];
     __shared__ double sm[33];
     if (bx == 0) {
-        const double rr = sum_partials(fslot(a, FP_RR), a.ntiles, sm);
-        const double bb = sum_partials(fslot(a, FP_BB), a.ntiles, sm);
-        const double tt = a.mixed ? sum_partials(fslot(a, FP_TT), a.ntiles, sm) : 0.0;
+        __shared__ double red[64];
+        double rr, tt = 0.0, bb = 0.0;
+        if (a.mixed)
+            partial_sums<2>(fslot(a, FP_RR), fslot(a, FP_TT), a.ntiles, red, &rr, &tt);
+        else
+            partial_sums<1>(fslot(a, FP_RR), nullptr, a.ntiles, red, &rr, nullptr);
+        if (a.st->target < 0) bb = sum_partials(fslot(a, FP_BB), a.ntiles, sm);  // first call
+        __syncthreads();  // (thread 0 sets the target)
         if (threadIdx.x == 0) {
             FpState *st = a.st;
             if (tick) st->k += 1;
@@ -605,15 +632,15 @@ __device__ __forceinline__ void k_fp_pre_blk(const FpArgs &a, int bx, int tick, 
             if (st->k >= a.maxiter && !st->done) st->done = 2;
         }
     }
-    const int H = a.smooth > 0 ? a.smooth : 1;
+    const int smooth = SM ? SM : a.smooth;
+    const int H = smooth > 0 ? smooth : 1;
     int mg[FP_MAXC];
     // sweep 1 from zero is pointwise: z = (omega / dg) r on the whole region
-    const int smooth = a.smooth;
     FpTile t = fp_tile(a, bx, H, fp_smem, mg, [&](int, int, int, bool, int, float wd, float r) {
         return smooth > 0 ? wd * r : 0.f;
     });
     __syncthreads();
-    const float *z = a.smooth > 1 ? fp_sweeps(t, mg, t.z0(), t.z1(), 0, a.smooth - 1) : t.z0();
+    const float *z = smooth > 1 ? fp_sweeps(t, mg, t.z0(), t.z1(), 0, smooth - 1) : t.z0();
     // this thread's tile cell
     const int lx = threadIdx.x & (FP_TILE - 1), ly = threadIdx.x / FP_TILE;
     const int row = H + ly, col = H + lx, l = row * t.R + col;
@@ -642,14 +669,20 @@ __device__ __forceinline__ void k_fp_pre_blk(const FpArgs &a, int bx, int tick, 
             for (int dy = 0; dy < f; ++dy)
                 for (int dx = 0; dx < f; ++dx)
                     sum += a.r1[(size_t)(gy + dy) * a.op.nx + gx + dx];
-            a.xin[2 * ((gy / f) * a.ncx + gx / f)] = (float)(sum / (f * f));
+            const int ic = (gy / f) * a.ncx + gx / f;
+            const float m = (float)(sum / (f * f));
+            if (net_next & 2)
+                a.out[ic] = m;
+            else
+                a.xin[2 * ic] = m;
         }
     }
 }
+template <int SM>
 __global__ void __launch_bounds__(CG_TILE, 2) k_fp_pre(FpArgs a, int tick, int net_next) {
     pdl_enter();
     FP_MEMBER(a);
-    k_fp_pre_blk(a, blockIdx.x, tick, net_next);
+    k_fp_pre_blk<SM>(a, blockIdx.x, tick, net_next);
 }
 
 // End of the preconditioner (one launch): z = `smooth` sweeps starting from
@@ -657,17 +690,19 @@ __global__ void __launch_bounds__(CG_TILE, 2) k_fp_pre(FpArgs a, int tick, int n
 // multiples of P y, c P y removes the most A-norm error from A d = r1, so the
 // network's correction can only help the smoothed iterate), written to a.z
 // with the partials <z_k, s_{k-1-j}> (j < min(k, m)) of the orthogonalisation.
+template <int SM>
 __device__ __forceinline__ void k_fp_post_blk(const FpArgs &a, int bx, int use_y) {
     __syncthreads();  // a previous call on this block has read its shared tile
     extern __shared__ __align__(16) unsigned char fp_smem[];
     __shared__ double sm[33];
     double c = 0.0;  // without the network's y this iteration: smoothing alone
     if (use_y) {
-        const double yr = sum_partials(fslot(a, FP_YR), a.ntiles, sm);
-        const double yay = sum_partials(fslot(a, FP_YAY), a.ntiles, sm);
+        __shared__ double red[64];
+        double yr, yay;
+        partial_sums<2>(fslot(a, FP_YR), fslot(a, FP_YAY), a.ntiles, red, &yr, &yay);
         c = yay > 0 ? yr / yay : 0.0;
     }
-    const int H = a.smooth;
+    const int H = SM ? SM : a.smooth;
     int mg[FP_MAXC];
     const int x0 = (bx % a.tx2) * FP_TILE - H, y0 = (bx / a.tx2) * FP_TILE - H;
     FpTile t = fp_tile(a, bx, H, fp_smem, mg, [&](int, int row, int col, bool in, int i, float, float) {
@@ -678,7 +713,7 @@ __device__ __forceinline__ void k_fp_post_blk(const FpArgs &a, int bx, int use_y
                   : 0.f;
     });
     __syncthreads();
-    const float *z = fp_sweeps(t, mg, t.z0(), t.z1(), 0, a.smooth);
+    const float *z = fp_sweeps(t, mg, t.z0(), t.z1(), 0, H);
     const int lx = threadIdx.x & (FP_TILE - 1), ly = threadIdx.x / FP_TILE;
     const int row = H + ly, col = H + lx, l = row * t.R + col;
     int i;
@@ -706,10 +741,11 @@ __device__ __forceinline__ void k_fp_post_blk(const FpArgs &a, int bx, int use_y
         if (threadIdx.x < nj) fslot(a, FP_ZS + threadIdx.x)[bx] = v[threadIdx.x];
     }
 }
+template <int SM>
 __global__ void __launch_bounds__(CG_TILE, 2) k_fp_post(FpArgs a, int use_y) {
     pdl_enter();
     FP_MEMBER(a);
-    k_fp_post_blk(a, blockIdx.x, use_y);
+    k_fp_post_blk<SM>(a, blockIdx.x, use_y);
 }
 
 size_t fp_smem_bytes(int H) { return 7 * sizeof(float) * (size_t)(FP_TILE + 2 * H) * (FP_TILE + 2 * H); }
@@ -720,18 +756,10 @@ __global__ void k_fp_wd(const float *dg32, float *wd32, int n) {
         wd32[i] = (float)(JACOBI_OMEGA / (double)dg32[i]);
 }
 
-// Identity in place of the network: out = R(r1) (unscaled; c absorbs the scale).
-__global__ void k_fp_identity(FpArgs a) {
-    pdl_enter();
-    const long long nall = (long long)a.nc * a.nmem;  // every member's coarse cells, one after the other
-    for (long long i = blockIdx.x * blockDim.x + threadIdx.x; i < nall; i += gridDim.x * blockDim.x)
-        a.out[i] = a.xin[2 * i];
-}
-
 // Partials <z, r1> and <z, A z> of the prolongated network output z = P y
 // (FP32 values, applied in FP64).
 __device__ __forceinline__ void k_fp_ydots_blk(const FpArgs &a, int bx) {
-    __shared__ double sm[33];
+    __shared__ double sm[64];
     const int i = bx * CG_TILE + threadIdx.x;
     double yr = 0, yay = 0;
     if (i < a.n) {
@@ -754,12 +782,7 @@ __device__ __forceinline__ void k_fp_ydots_blk(const FpArgs &a, int bx) {
         yr = __dmul_rn(zi, a.r1[i]);
         yay = __dmul_rn(zi, t);
     }
-    yr = block_sum(yr, sm);
-    yay = block_sum(yay, sm);
-    if (threadIdx.x == 0) {
-        fslot(a, FP_YR)[bx] = yr;
-        fslot(a, FP_YAY)[bx] = yay;
-    }
+    block_partials2(yr, yay, sm, fslot(a, FP_YR) + bx, fslot(a, FP_YAY) + bx);
 }
 __global__ void __launch_bounds__(CG_TILE) k_fp_ydots(FpArgs a) {
     pdl_enter();
@@ -821,6 +844,61 @@ __global__ void __launch_bounds__(CG_TILE) k_fp_dir(FpArgs a, cudaGraphCondition
     k_fp_dir_blk(a, blockIdx.x, cond, set_cond);
 }
 
+// k_fp_dir and the next iteration's k_fp_spmv in one kernel, for one direction kept (m =
+// 1): a row's neighbours' p_k are formed on the spot from z and p_{k-1} by their owners'
+// operation, so no launch lies between p_k and A p_k.
+__global__ void __launch_bounds__(CG_TILE, 2)
+    k_fp_dir_spmv(FpArgs a, cudaGraphConditionalHandle cond, int set_cond) {
+    pdl_enter();
+    FP_MEMBER(a);
+    __shared__ double sm[64];
+    const int k = (int)a.st->k, bx = blockIdx.x;
+    double beta = 0.0;
+    if (k > 0) {
+        double zs;
+        partial_sums<1>(fslot(a, FP_ZS), nullptr, a.ntiles2, sm, &zs, nullptr);
+        const double ps = a.st->ps[(k - 1) % a.ring];
+        beta = ps != 0.0 ? zs / ps : 0.0;
+        __syncthreads();
+    }
+    const size_t slot = (size_t)(k % a.ring) * a.sstride, old = (size_t)((k + 1) % a.ring) * a.sstride;
+    const StencilOp<2> &o = a.op;
+    const int i = bx * CG_TILE + threadIdx.x, nx = o.nx, iy = i / nx, ix = i - iy * nx;
+    double pr = 0.0, ps = 0.0;
+    if (i < a.n) {
+        if (a.mixed) {  // FP32 direction, beta rounded to FP32
+            const float bf = __double2float_rn(beta);
+            const float *po = a.pring32 + old, *z = a.z32;
+            auto p = [&](int j) { return k > 0 ? __fmaf_rn(-bf, po[j], z[j]) : z[j]; };
+            const float pi = p(i);
+            float t = __fmul_rn(o.dg32[i], pi);
+            if (ix > 0) t = __fmaf_rn(-o.we32[i - 1], p(i - 1), t);
+            if (ix < nx - 1) t = __fmaf_rn(-o.we32[i], p(i + 1), t);
+            if (iy > 0) t = __fmaf_rn(-o.wn32[i - nx], p(i - nx), t);
+            if (iy < o.ny - 1) t = __fmaf_rn(-o.wn32[i], p(i + nx), t);
+            a.pring32[slot + i] = pi;
+            a.sring32[slot + i] = t;
+            pr = xprod(pi, a.r32[i]);
+            ps = xprod(pi, t);
+        } else {
+            const double *po = a.pring + old, *z = a.z;
+            auto p = [&](int j) { return k > 0 ? __fma_rn(-beta, po[j], z[j]) : z[j]; };
+            const double pi = p(i);
+            double t = __dmul_rn(o.dg[i], pi);
+            if (ix > 0) t = __fma_rn(-o.we[i - 1], p(i - 1), t);
+            if (ix < nx - 1) t = __fma_rn(-o.we[i], p(i + 1), t);
+            if (iy > 0) t = __fma_rn(-o.wn[i - nx], p(i - nx), t);
+            if (iy < o.ny - 1) t = __fma_rn(-o.wn[i], p(i + nx), t);
+            a.pring[slot + i] = pi;
+            a.sring[slot + i] = t;
+            pr = __dmul_rn(pi, a.r[i]);
+            ps = __dmul_rn(pi, t);
+        }
+    }
+    block_partials2(pr, ps, sm, fslot(a, FP_PR) + bx, fslot(a, FP_PS) + bx);
+    if (set_cond && bx == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, a.st->done ? 0u : 1u);
+}
+
 // s_k = A p_k; partial <p_k, s_k>.
 __device__ __forceinline__ void k_fp_spmv_blk(const FpArgs &a, int bx) {
     __shared__ double sm[33];
@@ -846,8 +924,9 @@ __global__ void __launch_bounds__(CG_TILE) k_fp_spmv(FpArgs a) {
 // <p_k, s_k> kept in the ring for the orthogonalisations to come.
 __device__ __forceinline__ void k_fp_update_blk(const FpArgs &a, int bx) {
     __shared__ double sm[33];
-    const double ps = sum_partials(fslot(a, FP_PS), a.ntiles, sm);
-    const double pr = sum_partials(fslot(a, FP_PR), a.ntiles, sm);
+    __shared__ double red[64];
+    double ps, pr;
+    partial_sums<2>(fslot(a, FP_PS), fslot(a, FP_PR), a.ntiles, red, &ps, &pr);
     const int slot = (int)a.st->k % a.ring;
     const double alpha = ps != 0.0 ? pr / ps : 0.0;
     const int i = bx * CG_TILE + threadIdx.x;
@@ -862,7 +941,7 @@ __device__ __forceinline__ void k_fp_update_blk(const FpArgs &a, int bx) {
     if (threadIdx.x == 0) fslot(a, FP_RR)[bx] = rr;
     if (bx == 0 && threadIdx.x == 0) a.st->ps[slot] = ps;
 }
-__global__ void __launch_bounds__(CG_TILE) k_fp_update(FpArgs a) {
+__global__ void __launch_bounds__(CG_TILE, 2) k_fp_update(FpArgs a) {
     pdl_enter();
     FP_MEMBER(a);
     k_fp_update_blk(a, blockIdx.x);
@@ -937,8 +1016,9 @@ __global__ void __launch_bounds__(CG_TILE) k_fpm_spmv(FpArgs a) {
 // r32 -= alpha s (FP32); partial |r32|^2.
 __device__ __forceinline__ void k_fpm_update_blk(const FpArgs &a, int bx) {
     __shared__ double sm[33];
-    const double ps = sum_partials(fslot(a, FP_PS), a.ntiles, sm);
-    const double pr = sum_partials(fslot(a, FP_PR), a.ntiles, sm);
+    __shared__ double red[64];
+    double ps, pr;
+    partial_sums<2>(fslot(a, FP_PS), fslot(a, FP_PR), a.ntiles, red, &ps, &pr);
     const int slot = (int)a.st->k % a.ring;
     const float af = __double2float_rn(ps != 0.0 ? pr / ps : 0.0);
     float *d = fp_dm(a, a.st->par);
@@ -954,7 +1034,7 @@ __device__ __forceinline__ void k_fpm_update_blk(const FpArgs &a, int bx) {
     if (threadIdx.x == 0) fslot(a, FP_RR)[bx] = rr;
     if (bx == 0 && threadIdx.x == 0) a.st->ps[slot] = ps;
 }
-__global__ void __launch_bounds__(CG_TILE) k_fpm_update(FpArgs a) {
+__global__ void __launch_bounds__(CG_TILE, 2) k_fpm_update(FpArgs a) {
     pdl_enter();
     FP_MEMBER(a);
     k_fpm_update_blk(a, blockIdx.x);
@@ -1024,7 +1104,6 @@ enum FpPhaseCode : int {
     FPP_MUPDATE,
     FPP_MRELIABLE,
     FPP_PRE,       // x: tick, y: net_next
-    FPP_IDENTITY,  // the network's stand-in without a network: y = R r1
     FPP_YDOTS,
     FPP_POST,      // x: use_y
     FPP_DIR        // x: set the loop condition
@@ -1042,11 +1121,7 @@ __global__ void __launch_bounds__(CG_TILE, 2)
     k_fp_loop(const FpArgs a, const FpProgram pg, BarrierState *bar, cudaGraphConditionalHandle cond) {
     for (int s = 0; s < pg.n; ++s) {
         const int code = pg.op[s].code, ox = pg.op[s].x, oy = pg.op[s].y;
-        if (code == FPP_IDENTITY) {
-            for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.nc;
-                 i += (long long)gridDim.x * blockDim.x)
-                a.out[i] = a.xin[2 * i];
-        } else {
+        {
             const int nvb = (code == FPP_PRE || code == FPP_POST) ? a.ntiles2 : a.ntiles;
             for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
                 switch (code) {
@@ -1055,9 +1130,9 @@ __global__ void __launch_bounds__(CG_TILE, 2)
                     case FPP_MSPMV: k_fpm_spmv_blk(a, vb); break;
                     case FPP_MUPDATE: k_fpm_update_blk(a, vb); break;
                     case FPP_MRELIABLE: k_fpm_reliable_blk(a, vb); break;
-                    case FPP_PRE: k_fp_pre_blk(a, vb, ox, oy); break;
+                    case FPP_PRE: k_fp_pre_blk<0>(a, vb, ox, oy); break;
                     case FPP_YDOTS: k_fp_ydots_blk(a, vb); break;
-                    case FPP_POST: k_fp_post_blk(a, vb, ox); break;
+                    case FPP_POST: k_fp_post_blk<0>(a, vb, ox); break;
                     case FPP_DIR: k_fp_dir_blk(a, vb, cond, ox); break;
                     default: break;
                 }
@@ -1296,36 +1371,38 @@ int fp_network(cfm_fpcg *h, const FpArgs &a) {
 int fp_precond_dir(cfm_fpcg *h, const FpArgs &a, cudaGraphConditionalHandle cond, int set_cond, int tick,
                    bool use_net = true) {
     cudaStream_t s = h->stream;
-    const int net_next = !(h->net && !use_net);
+    const int net_next = !h->net ? 3 : use_net ? 1 : 0;
     const int M = h->nmem;
-    CFM_CUDA_TRY(launch_pdl(k_fp_pre, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(std::max(h->smooth, 1)),
-                            s, a, tick, net_next));
+    const auto pre = h->smooth == 4 ? k_fp_pre<4> : k_fp_pre<0>;
+    const auto post = h->smooth == 4 ? k_fp_post<4> : k_fp_post<0>;
+    const auto dir = h->m == 1 ? k_fp_dir_spmv : k_fp_dir;
+    CFM_CUDA_TRY(launch_pdl(pre, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(std::max(h->smooth, 1)), s, a,
+                            tick, net_next));
     if (!net_next) {
         // smoothing alone this iteration: no r1, no network, c = 0
-        CFM_CUDA_TRY(launch_pdl(k_fp_post, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(h->smooth), s, a, 0));
-        CFM_CUDA_TRY(launch_pdl(k_fp_dir, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a, cond, set_cond));
+        CFM_CUDA_TRY(launch_pdl(post, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(h->smooth), s, a, 0));
+        CFM_CUDA_TRY(launch_pdl(dir, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a, cond, set_cond));
         return CFM_OK;
     }
     if (h->net) {
         const int st = fp_network(h, a);
         if (st) return st;
-    } else {
-        CFM_CUDA_TRY(launch_pdl(k_fp_identity, dim3(256), dim3(256), 0, s, a));
     }
     CFM_CUDA_TRY(launch_pdl(k_fp_ydots, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a));
-    CFM_CUDA_TRY(launch_pdl(k_fp_post, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(h->smooth), s, a, 1));
-    CFM_CUDA_TRY(launch_pdl(k_fp_dir, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a, cond, set_cond));
+    CFM_CUDA_TRY(launch_pdl(post, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(h->smooth), s, a, 1));
+    CFM_CUDA_TRY(launch_pdl(dir, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a, cond, set_cond));
     return CFM_OK;
 }
 
 int fp_iteration(cfm_fpcg *h, const FpArgs &a, cudaGraphConditionalHandle cond, int set_cond, bool use_net) {
     const dim3 g(h->ntiles, h->nmem);
+    // (with m = 1 the direction kernel before has left A p)
     if (h->mixed) {
-        CFM_CUDA_TRY(launch_pdl(k_fpm_spmv, g, dim3(CG_TILE), 0, h->stream, a));
+        if (h->m > 1) CFM_CUDA_TRY(launch_pdl(k_fpm_spmv, g, dim3(CG_TILE), 0, h->stream, a));
         CFM_CUDA_TRY(launch_pdl(k_fpm_update, g, dim3(CG_TILE), 0, h->stream, a));
         CFM_CUDA_TRY(launch_pdl(k_fpm_reliable, g, dim3(CG_TILE), 0, h->stream, a));
     } else {
-        CFM_CUDA_TRY(launch_pdl(k_fp_spmv, g, dim3(CG_TILE), 0, h->stream, a));
+        if (h->m > 1) CFM_CUDA_TRY(launch_pdl(k_fp_spmv, g, dim3(CG_TILE), 0, h->stream, a));
         CFM_CUDA_TRY(launch_pdl(k_fp_update, g, dim3(CG_TILE), 0, h->stream, a));
     }
     return fp_precond_dir(h, a, cond, set_cond, 1, use_net);
@@ -1379,7 +1456,7 @@ int fp_body_loop(cfm_fpcg *h, const FpArgs &a, cudaGraphConditionalHandle cond, 
     };
     for (int j = 0; j < h->net_every; ++j) {
         const int set = set_cond && j == h->net_every - 1;
-        const int net_next = !(h->net && j != 0);
+        const int net_next = !h->net ? 3 : j == 0 ? 1 : 0;
         if ((st = add(h->mixed ? FPP_MSPMV : FPP_SPMV, 0, 0)) || (st = add(h->mixed ? FPP_MUPDATE : FPP_UPDATE, 0, 0)))
             return st;
         if (h->mixed && (st = add(FPP_MRELIABLE, 0, 0))) return st;
@@ -1390,8 +1467,6 @@ int fp_body_loop(cfm_fpcg *h, const FpArgs &a, cudaGraphConditionalHandle cond, 
         }
         if (h->net) {
             if ((st = fp_loop_launch(h, a, pg, cond)) || (st = fp_network(h, a))) return st;
-        } else if ((st = add(FPP_IDENTITY, 0, 0))) {
-            return st;
         }
         if ((st = add(FPP_YDOTS, 0, 0)) || (st = add(FPP_POST, 1, 0)) || (st = add(FPP_DIR, set, 0))) return st;
     }
@@ -1491,13 +1566,21 @@ int fp_setup(cfm_fpcg *h, int nx, int ny, int f, cfm_unet *net, int smooth, int 
         (e = cudaMalloc(&h->xin, sizeof(float) * 2 * (size_t)h->nc * nmem)) != cudaSuccess ||
         (e = cudaMalloc(&h->out, sizeof(float) * (size_t)h->nc * nmem)) != cudaSuccess ||
         (e = cudaMalloc(&h->part, sizeof(double) * FP_NSLOT * (size_t)h->pstride * nmem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_pre, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (e = cudaFuncSetAttribute(k_fp_pre<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_post, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (e = cudaFuncSetAttribute(k_fp_pre<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_pre, cudaFuncAttributePreferredSharedMemoryCarveout,
+        (e = cudaFuncSetAttribute(k_fp_post<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(k_fp_post<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(k_fp_pre<0>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_post, cudaFuncAttributePreferredSharedMemoryCarveout,
+        (e = cudaFuncSetAttribute(k_fp_pre<4>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(k_fp_post<0>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(k_fp_post<4>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
         (e = cudaMalloc(&h->acc, sizeof(double) * std::max(4, nmem))) != cudaSuccess ||
         (e = cudaMalloc(&h->rslots, sizeof(double) * FP_RES_BLOCKS * (size_t)nmem)) != cudaSuccess ||
