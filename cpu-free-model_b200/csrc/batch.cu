@@ -23,7 +23,9 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include "barrier.cuh"
@@ -34,7 +36,8 @@ namespace cfm {
 
 namespace {
 
-constexpr int BT_MAXCLS = 4;
+constexpr int BT_MAXCLS = 8;   // classes of a launch
+constexpr int BT_PLANCLS = 4;  // classes of a caller's plan
 constexpr double BT_OMEGA = 0.8;
 
 struct BtSys {
@@ -647,7 +650,7 @@ struct cfm_batch {
     int ncls = 0, blocks = 0, nteams = 0;
     int cls_team[BT_MAXCLS] = {}, cls_block0[BT_MAXCLS] = {}, cls_team0[BT_MAXCLS] = {};
     int cls_start[BT_MAXCLS] = {}, cls_count[BT_MAXCLS] = {};
-    long long thr[BT_MAXCLS] = {};
+    bool own_plan = false;  // auto_plan's, not the caller's
     int smooth = 4, maxiter = 20000;
     double tol = 1e-8;
     // FP32 iteration with FP64 reliable updates
@@ -672,59 +675,31 @@ void drop_graph(cfm_batch *h) {
     }
 }
 
-// Classes by size: class c holds systems with n >= thr[c] (thr descending,
-// thr[ncls-1] = 0); blocks are shared out in proportion to each class's
-// work estimate sum(n * side), rounded to whole teams.
-int plan(cfm_batch *h, int ncls, const long long *thr, const int *team, int blocks) {
-    CFM_ARG_CHECK(ncls >= 1 && ncls <= BT_MAXCLS, "classes");
-    std::vector<int> idx(h->nsys);
-    std::iota(idx.begin(), idx.end(), 0);
-    std::sort(idx.begin(), idx.end(), [&](int x, int y) { return h->sys[x].n > h->sys[y].n; });
+// A division of the systems into classes: per class the team size, the number of teams
+// and the systems in queue order.
+struct BtPlan {
+    struct Class {
+        int team = 0, teams = 0;
+        std::vector<int> sys;
+    };
+    std::vector<Class> cls;
+};
+
+// Takes over a plan.
+int install_plan(cfm_batch *h, const BtPlan &p) {
     std::vector<int> order;
-    std::vector<double> work(ncls, 0.0);
-    int start = 0;
-    for (int c = 0; c < ncls; ++c) {
-        h->cls_start[c] = start;
-        int cnt = 0;
-        for (int i : idx) {
-            const long long n = h->sys[i].n;
-            const bool in = n >= thr[c] && (c == 0 || n < thr[c - 1]);
-            if (!in) continue;
-            order.push_back(i);
-            ++cnt;
-            const BtSys &S = h->sys[i];
-            const double side = S.dims == 3 ? std::cbrt((double)n) : std::sqrt((double)n);
-            work[c] += (double)n * side;
-        }
-        h->cls_count[c] = cnt;
-        start += cnt;
+    h->ncls = (int)p.cls.size();
+    h->blocks = h->nteams = 0;
+    for (int c = 0; c < h->ncls; ++c) {
+        h->cls_start[c] = (int)order.size();
+        h->cls_count[c] = (int)p.cls[c].sys.size();
+        h->cls_team[c] = p.cls[c].team;
+        h->cls_block0[c] = h->blocks;
+        h->cls_team0[c] = h->nteams;
+        h->blocks += p.cls[c].team * p.cls[c].teams;
+        h->nteams += p.cls[c].teams;
+        order.insert(order.end(), p.cls[c].sys.begin(), p.cls[c].sys.end());
     }
-    CFM_ARG_CHECK((int)order.size() == h->nsys, "class thresholds must cover every system");
-    const double wsum = std::accumulate(work.begin(), work.end(), 0.0);
-    int b0 = 0, t0 = 0;
-    for (int c = 0; c < ncls; ++c) {
-        int nb;
-        if (c == ncls - 1) {
-            nb = blocks - b0;
-        } else {
-            nb = (int)std::lround(blocks * (wsum > 0 ? work[c] / wsum : 1.0 / ncls));
-        }
-        nb = std::max(h->cls_count[c] > 0 ? team[c] : 0, nb / team[c] * team[c]);
-        if (b0 + nb > blocks) nb = (blocks - b0) / team[c] * team[c];
-        if (h->cls_count[c] > 0 && nb < team[c]) {
-            set_error("not enough resident blocks for the class plan");
-            return CFM_UNSUPPORTED;
-        }
-        h->cls_team[c] = team[c];
-        h->cls_block0[c] = b0;
-        h->cls_team0[c] = t0;
-        b0 += nb;
-        t0 += nb / team[c];
-        h->thr[c] = thr[c];
-    }
-    h->ncls = ncls;
-    h->blocks = b0;
-    h->nteams = t0;
     drop_graph(h);
     if (h->order) cudaFree(h->order);
     if (h->bars) cudaFree(h->bars);
@@ -737,6 +712,160 @@ int plan(cfm_batch *h, int ncls, const long long *thr, const int *team, int bloc
     CFM_CUDA_TRY(cudaMalloc(&h->team_sys, sizeof(int) * std::max(1, h->nteams)));
     CFM_CUDA_TRY(cudaMemcpy(h->order, order.data(), sizeof(int) * h->nsys, cudaMemcpyHostToDevice));
     return CFM_OK;
+}
+
+double bt_side(const BtSys &S) { return S.dims == 3 ? std::cbrt((double)S.n) : std::sqrt((double)S.n); }
+
+// Classes by size: class c holds systems with n >= thr[c] (thr descending,
+// thr[ncls-1] = 0); blocks are shared out in proportion to each class's
+// work estimate sum(n * side), rounded to whole teams.  False when the blocks do not
+// suffice.
+bool threshold_plan(const cfm_batch *h, int ncls, const long long *thr, const int *team, int blocks, BtPlan *p) {
+    std::vector<int> idx(h->nsys);
+    std::iota(idx.begin(), idx.end(), 0);
+    std::sort(idx.begin(), idx.end(), [&](int x, int y) { return h->sys[x].n > h->sys[y].n; });
+    p->cls.assign(ncls, BtPlan::Class());
+    std::vector<double> work(ncls, 0.0);
+    for (int i : idx) {
+        int c = 0;
+        while (c + 1 < ncls && h->sys[i].n < thr[c]) ++c;
+        p->cls[c].sys.push_back(i);
+        work[c] += (double)h->sys[i].n * bt_side(h->sys[i]);
+    }
+    const double wsum = std::accumulate(work.begin(), work.end(), 0.0);
+    int b0 = 0;
+    for (int c = 0; c < ncls; ++c) {
+        int nb = c == ncls - 1 ? blocks - b0
+                               : (int)std::lround(blocks * (wsum > 0 ? work[c] / wsum : 1.0 / ncls));
+        nb = std::max(!p->cls[c].sys.empty() ? team[c] : 0, nb / team[c] * team[c]);
+        if (b0 + nb > blocks) nb = (blocks - b0) / team[c] * team[c];
+        if (!p->cls[c].sys.empty() && nb < team[c]) return false;
+        p->cls[c].team = team[c];
+        p->cls[c].teams = nb / team[c];
+        b0 += nb;
+    }
+    return true;
+}
+
+// Threshold plans that the autotuner times and the starting plan considers.
+struct BtCand {
+    int ncls;
+    long long thr[BT_PLANCLS];
+    int team[BT_PLANCLS];
+};
+const BtCand bt_cands[] = {
+    {3, {1LL << 18, 1LL << 15, 0}, {16, 4, 1}},
+    {3, {1LL << 18, 1LL << 15, 0}, {8, 2, 1}},
+    {3, {1LL << 19, 1LL << 16, 0}, {32, 4, 1}},
+    {3, {1LL << 17, 1LL << 14, 0}, {8, 2, 1}},
+    {2, {1LL << 16, 0}, {8, 1}},
+    {4, {1LL << 19, 1LL << 17, 1LL << 14, 0}, {32, 8, 2, 1}},
+};
+
+// The plan a batch starts with: of the threshold plans and of two fitted to the batch, the
+// one with the shortest modelled launch.  A team of T blocks takes about
+//   iterations x passes x (sync + ceil(tiles / T) x tile)
+// for a system: iterations in proportion to its side, sync 0.5 us for one block and 2 us
+// behind a team barrier, tile 0.57 us while the systems being solved fit in L2 and up to
+// 0.98 us when they are ten times as large (B200, one 1024-row tile in one pass).  So large
+// batches want few, wide teams, and small ones want every block busy: by thresholds alone
+// a batch of 30 systems of up to 457^2 ran on teams of four blocks and 60% of the chip
+// idled (FP32 213 ms, 64 ms with the fitted plan).
+int auto_plan(cfm_batch *h, int blocks) {
+    const int sizes[BT_MAXCLS] = {64, 48, 32, 16, 8, 4, 2, 1};
+    const double cell = h->mixed ? 40.0 : 80.0;  // bytes per cell that an iteration goes through
+    const int nsys = h->nsys;
+    double tile = 0.57;
+    auto time = [&](int i, int T) {
+        return bt_side(h->sys[i]) * ((T == 1 ? 0.5 : 2.0) + tile * ((h->sys[i].ntiles + T - 1) / T));
+    };
+    // end of a class's queue: its systems in order, each to the team that is free first
+    auto queue_end = [&](const BtPlan::Class &c, int teams) {
+        std::priority_queue<double, std::vector<double>, std::greater<double>> end;
+        for (int q = 0; q < teams; ++q) end.push(0.0);
+        double last = 0;
+        for (int i : c.sys) {
+            const double e = end.top() + time(i, c.team);
+            end.pop();
+            end.push(e);
+            last = std::max(last, e);
+        }
+        return last;
+    };
+    auto length = [&](const BtPlan &p) {
+        double foot = 0, last = 0;
+        for (const auto &c : p.cls) {
+            if (c.sys.empty()) continue;
+            double cells = 0;
+            for (int i : c.sys) cells += h->sys[i].n;
+            foot += cell * cells / c.sys.size() * std::min<size_t>(c.teams, c.sys.size());
+        }
+        tile = 0.57 + 0.41 * std::min(1.0, std::max(0.0, (foot - 100e6) / 1100e6));
+        for (const auto &c : p.cls)
+            if (!c.sys.empty()) last = std::max(last, queue_end(c, c.teams));
+        return last;
+    };
+    std::vector<int> idx(nsys);
+    std::iota(idx.begin(), idx.end(), 0);
+    std::sort(idx.begin(), idx.end(), [&](int x, int y) {
+        return h->sys[x].n * bt_side(h->sys[x]) > h->sys[y].n * bt_side(h->sys[y]);
+    });
+    // The fitted plan for a length: each system gets the widest team that leaves it `least`
+    // tiles per block, or a wider one that solves it in time, and each class as few teams
+    // as end in time.  False when the blocks do not suffice.
+    auto fit = [&](double len, long long least, BtPlan *p) {
+        p->cls.clear();
+        std::vector<BtPlan::Class> by(BT_MAXCLS);
+        for (int i : idx) {
+            int c = BT_MAXCLS - 1;
+            while (c > 0 && sizes[c - 1] <= blocks && h->sys[i].ntiles >= least * sizes[c - 1]) --c;
+            while (c > 0 && sizes[c - 1] <= blocks && time(i, sizes[c]) > len) --c;
+            if (time(i, sizes[c]) > len) return false;
+            by[c].team = sizes[c];
+            by[c].sys.push_back(i);
+        }
+        int used = 0;
+        for (auto &c : by) {
+            if (c.sys.empty()) continue;
+            double sum = 0;
+            for (int i : c.sys) sum += time(i, c.team);
+            c.teams = std::max(1, (int)(sum / len));
+            while (used + c.teams * c.team <= blocks && queue_end(c, c.teams) > len) ++c.teams;
+            used += c.teams * c.team;
+            if (used > blocks) return false;
+            p->cls.push_back(c);
+        }
+        return true;
+    };
+    BtPlan best, p;
+    double best_len = 1e300;
+    auto consider = [&]() {
+        const double l = length(p);
+        if (l < best_len) {
+            best_len = l;
+            best = p;
+        }
+    };
+    for (const BtCand &c : bt_cands)
+        if (threshold_plan(h, c.ncls, c.thr, c.team, blocks, &p)) consider();
+    for (long long least : {1LL << 40, 64LL}) {
+        tile = 0.57;
+        double lo = 0, hi = 0;
+        for (int i = 0; i < nsys; ++i) hi += time(i, 1) + time(i, 2);
+        if (!fit(hi, least, &p)) continue;
+        for (int it = 0; it < 24 && hi - lo > 1e-3 * hi; ++it) {
+            const double mid = 0.5 * (lo + hi);
+            (fit(mid, least, &p) ? hi : lo) = mid;
+        }
+        fit(hi, least, &p);
+        consider();
+    }
+    if (best.cls.empty()) {
+        set_error("not enough resident blocks for the class plan");
+        return CFM_UNSUPPORTED;
+    }
+    h->own_plan = true;
+    return install_plan(h, best);
 }
 
 BtArgs bt_args(cfm_batch *h) {
@@ -930,16 +1059,13 @@ int cfm_batch_create(int nsys, const int *dims, const int *nx, const int *ny, co
             cudaSuccess)
             return fail(e);
     }
-    // default plan: three classes, team sizes 16 / 4 / 1
     int blocks = 0;
     int st = resident_blocks(&blocks);
     if (st) {
         cfm_batch_destroy(h);
         return st;
     }
-    const long long thr[3] = {1LL << 18, 1LL << 15, 0};
-    const int team[3] = {16, 4, 1};
-    if ((st = plan(h, 3, thr, team, blocks))) {
+    if ((st = auto_plan(h, blocks))) {
         cfm_batch_destroy(h);
         return st;
     }
@@ -979,7 +1105,18 @@ int cfm_batch_set_plan(cfm_batch *h, int ncls, const long long *thresholds, cons
     int blocks = 0;
     int st = resident_blocks(&blocks);
     if (st) return st;
-    return plan(h, ncls, thresholds, team_sizes, blocks);
+    CFM_ARG_CHECK(ncls >= 1 && ncls <= BT_PLANCLS, "classes");
+    long long placed = 0;  // thresholds that do not descend leave systems out or twice in
+    for (const BtSys &S : h->sys)
+        for (int c = 0; c < ncls; ++c) placed += S.n >= thresholds[c] && (c == 0 || S.n < thresholds[c - 1]);
+    CFM_ARG_CHECK(placed == h->nsys, "class thresholds must cover every system");
+    BtPlan p;
+    if (!threshold_plan(h, ncls, thresholds, team_sizes, blocks, &p)) {
+        set_error("not enough resident blocks for the class plan");
+        return CFM_UNSUPPORTED;
+    }
+    h->own_plan = false;
+    return install_plan(h, p);
 }
 
 int cfm_batch_set_solver(cfm_batch *h, int smooth, int maxiter, double tol) {
@@ -1013,10 +1150,16 @@ int cfm_batch_set_precision(cfm_batch *h, int precision, int inner_maxiter, doub
         CFM_CUDA_TRY(cudaGetLastError());
         CFM_CUDA_TRY(cudaStreamSynchronize(h->stream));
     }
+    const bool changed = h->mixed != (precision == CFM_FP32);
     h->mixed = precision == CFM_FP32;
     h->inner_maxiter = inner_maxiter;
     h->inner_tol = inner_tol > 0 ? inner_tol : 0.1;
     drop_graph(h);
+    if (changed && h->own_plan) {  // the working set is another
+        int blocks = 0;
+        const int st = resident_blocks(&blocks);
+        return st ? st : auto_plan(h, blocks);
+    }
     return CFM_OK;
 }
 
@@ -1077,23 +1220,18 @@ int cfm_batch_autotune(cfm_batch *h, double *best_ms) {
     const cfm::NvtxRange nvtx_range("cfm_batch_autotune");
     clear_error();
     CFM_ARG_CHECK(h, "null argument");
-    struct Cand {
-        int ncls;
-        long long thr[BT_MAXCLS];
-        int team[BT_MAXCLS];
-    };
-    const Cand cands[] = {
-        {3, {1LL << 18, 1LL << 15, 0}, {16, 4, 1}},
-        {3, {1LL << 18, 1LL << 15, 0}, {8, 2, 1}},
-        {3, {1LL << 19, 1LL << 16, 0}, {32, 4, 1}},
-        {3, {1LL << 17, 1LL << 14, 0}, {8, 2, 1}},
-        {2, {1LL << 16, 0}, {8, 1}},
-        {4, {1LL << 19, 1LL << 17, 1LL << 14, 0}, {32, 8, 2, 1}},
-    };
     double best = 1e300;
-    int bi = -1;
-    for (int c = 0; c < (int)(sizeof(cands) / sizeof(cands[0])); ++c) {
-        if (cfm_batch_set_plan(h, cands[c].ncls, cands[c].thr, cands[c].team) != CFM_OK) continue;
+    int bi = -1;  // -1: the plan a batch starts with
+    int blocks = 0;
+    int st = resident_blocks(&blocks);
+    if (st || (st = auto_plan(h, blocks))) return st;
+    {
+        float ms = 0;
+        if ((st = run_once(h, &ms))) return st;
+        best = ms;
+    }
+    for (int c = 0; c < (int)(sizeof(bt_cands) / sizeof(bt_cands[0])); ++c) {
+        if (cfm_batch_set_plan(h, bt_cands[c].ncls, bt_cands[c].thr, bt_cands[c].team) != CFM_OK) continue;
         float ms = 0;
         int e = run_once(h, &ms);
         if (e) return e;
@@ -1102,8 +1240,7 @@ int cfm_batch_autotune(cfm_batch *h, double *best_ms) {
             bi = c;
         }
     }
-    CFM_ARG_CHECK(bi >= 0, "no candidate plan fits this device");
-    int st = cfm_batch_set_plan(h, cands[bi].ncls, cands[bi].thr, cands[bi].team);
+    st = bi < 0 ? auto_plan(h, blocks) : cfm_batch_set_plan(h, bt_cands[bi].ncls, bt_cands[bi].thr, bt_cands[bi].team);
     if (st) return st;
     if (best_ms) *best_ms = best;
     return CFM_OK;

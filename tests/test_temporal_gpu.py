@@ -142,3 +142,21 @@ def test_cg_many_tiles_repeated():
             x, st = h.solve(b)
             assert st.iterations == it_o
             np.testing.assert_array_equal(x, xo)
+
+
+def test_batch_starting_plan_covers_every_system():
+    """The plan a batch starts with (team sizes from 1 to 64 blocks side by side) solves
+    every system to the same bits as one team size for all."""
+    systems = [cfm.varcoef_problem(s, 40 + i) for i, s in
+               enumerate([(300, 300), (16, 16), (64, 70), (40, 40, 40), (9, 9, 9), (128, 128), (33, 1), (200, 210)])]
+    for prec in (cfm.FP64, cfm.FP32):
+        B = cfm.Batch(systems)
+        B.set_precision(prec)
+        it0, st0, rr0, _ = B.solve()
+        xs = [B.solution(i) for i in range(B.n)]
+        assert (st0 == cfm.OK).all() and (rr0 <= 1e-8).all()
+        B.set_plan([0], [4])
+        it1, st1, _, _ = B.solve()
+        assert (it0 == it1).all() and (st0 == st1).all()
+        for i in range(B.n):
+            np.testing.assert_array_equal(B.solution(i), xs[i])
