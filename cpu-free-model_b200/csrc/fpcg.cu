@@ -581,59 +581,60 @@ __device__ __forceinline__ float *fp_sweeps(const FpTile &t, const int *mg, floa
     return cur;
 }
 
+// The iteration's bookkeeping (one block of NW warps): [k += 1 when `tick`]; |r|^2
+// history, convergence / stall test.
+template <int NW>
+__device__ __forceinline__ void fp_pre_state(const FpArgs &a, int tick) {
+    __shared__ double red[64], redb[32];
+    double rr, tt = 0.0, bb = 0.0;
+    if (a.mixed)
+        partial_sums<2, NW>(fslot(a, FP_RR), fslot(a, FP_TT), a.ntiles, red, &rr, &tt);
+    else
+        partial_sums<1, NW>(fslot(a, FP_RR), nullptr, a.ntiles, red, &rr, nullptr);
+    if (a.st->target < 0) partial_sums<1, NW>(fslot(a, FP_BB), nullptr, a.ntiles, redb, &bb, nullptr);  // first call
+    __syncthreads();  // (thread 0 sets the target)
+    if (threadIdx.x == 0) {
+        FpState *st = a.st;
+        if (tick) st->k += 1;
+        double target = st->target;
+        if (target < 0) {  // first call: target = tol * |b|
+            target = -target * sqrt(bb);
+            st->target = target;
+        }
+        if (st->k <= a.maxiter) a.hist[st->k] = sqrt(rr);
+        if (!a.mixed) {
+            if (sqrt(rr) <= target) st->done = 1;
+        } else if (st->pending) {  // a reliable update ran: the FP64 true residual judges
+            st->par ^= 1;
+            st->pending = 0;
+            st->updates += 1;
+            st->gmax = rr;
+            if (sqrt(tt) <= target) st->done = 1;
+        } else if (rr > st->gmax) {
+            st->gmax = rr;
+        }
+        if (rr < st->best_rr) {
+            st->best_rr = rr;
+            st->best_k = st->k;
+        } else if (st->k - st->best_k > a.stall) {
+            st->done = 2;
+        }
+        if (st->k >= a.maxiter && !st->done) st->done = 2;
+    }
+}
+
 // Start of the preconditioner (one launch): [k += 1 when `tick`; block 0:
 // |r|^2 history, convergence / stall test]; z0 = `smooth` sweeps from zero
 // and, when the network follows (`net_next`), r1 = r - A z0, partial
 // |r1|^2, and the network input channel 0 = R(r1) (f x f means; the network
 // scales it by 1 / rms(r1) itself).  net_next & 2: R(r1) goes to the network's output
 // instead (no network: the identity stands in, and c absorbs the scale).
-// SM: the sweeps when known at compile time (the region's divisions and strides are
-// constants then; k_fp_pre<4> and k_fp_post<4> serve the default depth), else 0.
-template <int SM>
 __device__ __forceinline__ void k_fp_pre_blk(const FpArgs &a, int bx, int tick, int net_next) {
     __syncthreads();  // a previous call on this block has read its shared tile
     extern __shared__ __align__(16) unsigned char fp_smem[];
     __shared__ double sm[33];
-    if (bx == 0) {
-        __shared__ double red[64];
-        double rr, tt = 0.0, bb = 0.0;
-        if (a.mixed)
-            partial_sums<2>(fslot(a, FP_RR), fslot(a, FP_TT), a.ntiles, red, &rr, &tt);
-        else
-            partial_sums<1>(fslot(a, FP_RR), nullptr, a.ntiles, red, &rr, nullptr);
-        if (a.st->target < 0) bb = sum_partials(fslot(a, FP_BB), a.ntiles, sm);  // first call
-        __syncthreads();  // (thread 0 sets the target)
-        if (threadIdx.x == 0) {
-            FpState *st = a.st;
-            if (tick) st->k += 1;
-            double target = st->target;
-            if (target < 0) {  // first call: target = tol * |b|
-                target = -target * sqrt(bb);
-                st->target = target;
-            }
-            if (st->k <= a.maxiter) a.hist[st->k] = sqrt(rr);
-            if (!a.mixed) {
-                if (sqrt(rr) <= target) st->done = 1;
-            } else if (st->pending) {  // a reliable update ran: the FP64 true residual judges
-                st->par ^= 1;
-                st->pending = 0;
-                st->updates += 1;
-                st->gmax = rr;
-                if (sqrt(tt) <= target) st->done = 1;
-            } else if (rr > st->gmax) {
-                st->gmax = rr;
-            }
-            if (rr < st->best_rr) {
-                st->best_rr = rr;
-                st->best_k = st->k;
-            } else if (st->k - st->best_k > a.stall) {
-                st->done = 2;
-            }
-            if (st->k >= a.maxiter && !st->done) st->done = 2;
-        }
-    }
-    const int smooth = SM ? SM : a.smooth;
-    const int H = smooth > 0 ? smooth : 1;
+    if (bx == 0) fp_pre_state<32>(a, tick);
+    const int smooth = a.smooth, H = smooth > 0 ? smooth : 1;
     int mg[FP_MAXC];
     // sweep 1 from zero is pointwise: z = (omega / dg) r on the whole region
     FpTile t = fp_tile(a, bx, H, fp_smem, mg, [&](int, int, int, bool, int, float wd, float r) {
@@ -678,11 +679,10 @@ __device__ __forceinline__ void k_fp_pre_blk(const FpArgs &a, int bx, int tick, 
         }
     }
 }
-template <int SM>
 __global__ void __launch_bounds__(CG_TILE, 2) k_fp_pre(FpArgs a, int tick, int net_next) {
     pdl_enter();
     FP_MEMBER(a);
-    k_fp_pre_blk<SM>(a, blockIdx.x, tick, net_next);
+    k_fp_pre_blk(a, blockIdx.x, tick, net_next);
 }
 
 // End of the preconditioner (one launch): z = `smooth` sweeps starting from
@@ -690,11 +690,9 @@ __global__ void __launch_bounds__(CG_TILE, 2) k_fp_pre(FpArgs a, int tick, int n
 // multiples of P y, c P y removes the most A-norm error from A d = r1, so the
 // network's correction can only help the smoothed iterate), written to a.z
 // with the partials <z_k, s_{k-1-j}> (j < min(k, m)) of the orthogonalisation.
-template <int SM>
 __device__ __forceinline__ void k_fp_post_blk(const FpArgs &a, int bx, int use_y) {
     __syncthreads();  // a previous call on this block has read its shared tile
     extern __shared__ __align__(16) unsigned char fp_smem[];
-    __shared__ double sm[33];
     double c = 0.0;  // without the network's y this iteration: smoothing alone
     if (use_y) {
         __shared__ double red[64];
@@ -702,7 +700,7 @@ __device__ __forceinline__ void k_fp_post_blk(const FpArgs &a, int bx, int use_y
         partial_sums<2>(fslot(a, FP_YR), fslot(a, FP_YAY), a.ntiles, red, &yr, &yay);
         c = yay > 0 ? yr / yay : 0.0;
     }
-    const int H = SM ? SM : a.smooth;
+    const int H = a.smooth;
     int mg[FP_MAXC];
     const int x0 = (bx % a.tx2) * FP_TILE - H, y0 = (bx / a.tx2) * FP_TILE - H;
     FpTile t = fp_tile(a, bx, H, fp_smem, mg, [&](int, int row, int col, bool in, int i, float, float) {
@@ -741,11 +739,245 @@ __device__ __forceinline__ void k_fp_post_blk(const FpArgs &a, int bx, int use_y
         if (threadIdx.x < nj) fslot(a, FP_ZS + threadIdx.x)[bx] = v[threadIdx.x];
     }
 }
-template <int SM>
 __global__ void __launch_bounds__(CG_TILE, 2) k_fp_post(FpArgs a, int use_y) {
     pdl_enter();
     FP_MEMBER(a);
-    k_fp_post_blk<SM>(a, blockIdx.x, use_y);
+    k_fp_post_blk(a, blockIdx.x, use_y);
+}
+
+// The same two launches at the default depth of FS_H = 4 sweeps, with a tile's cells in
+// registers: a thread holds FS_H cells of one column of the 40 x 40 region and the seven
+// operator and right-hand side words of each, loaded once and straight from global memory;
+// only the iterate goes through shared memory (double-buffered, one block barrier per
+// sweep), since neighbours need it.  The general kernels read 12 shared words for each
+// cell and sweep and test every cell's margin: instruction-bound at 512^2 (256 tiles, two
+// on most SMs).  FPCG without a network, per iteration, the general kernels at a compile-time
+// depth against these: 64^2 31.8 / 28.3 us, 512^2 43.6 / 38.0, 700^2 80.1 / 67.8.  What is
+// left is latency: two block-wide hand-overs of sums, one trip to L2, a barrier per sweep.
+// Other depths (and the device loop, whose blocks have 1024 threads) take the general
+// kernels.  Cells outside a sweep's valid margin are updated here as well, from
+// whatever is beside them, and never reach a valid cell.  Every valid cell and every dot
+// is formed by the same operations in the same order as there.  The row stride of 42 words
+// puts a warp's 32 cells, which can straddle two strips, in 32 banks.
+constexpr int FS_H = 4, FS_R = FP_TILE + 2 * FS_H, FS_LD = 42, FS_NW = 16;
+constexpr int FS_ACTIVE = FS_R * (FS_R / FS_H);  // threads that hold cells
+static_assert(FS_R % FS_H == 0 && FS_ACTIVE <= 32 * FS_NW && FP_TILE % FS_NW == 0, "strips and dot rows");
+static_assert((FS_H * FS_LD - FS_R) % 32 == 0, "consecutive threads in consecutive banks");
+
+struct FpStrip {
+    float r[FS_H], dg[FS_H], wd[FS_H], we[FS_H], wl[FS_H], wn[FS_H + 1];  // wl: the face to x - 1
+    float u[FS_H];
+    bool in[FS_H];
+    int i, nx;  // global index of the first cell
+    float *own, *left, *right, *up, *down;  // of the first cell in buffer 0; beside and around the strip
+
+    // Loads the strip of thread t < FS_ACTIVE of tile bx (zeros outside the grid, as fp_tile).
+    __device__ __forceinline__ void load(const FpArgs &a, int bx, float *buf, int t) {
+        const int s = t / FS_R, col = t - s * FS_R;
+        const int gx = (bx % a.tx2) * FP_TILE - FS_H + col, gy = (bx / a.tx2) * FP_TILE - FS_H + s * FS_H;
+        nx = a.op.nx;
+        i = gy * nx + gx;
+        const bool inx = gx >= 0 && gx < nx;
+        wn[0] = inx && gy > 0 && gy - 1 < a.op.ny ? a.wn32[i - nx] : 0.f;
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) {
+            const int j = i + k * nx;
+            in[k] = inx && gy + k >= 0 && gy + k < a.op.ny;
+            r[k] = in[k] ? (a.mixed ? a.r32[j] : (float)a.r[j]) : 0.f;
+            we[k] = in[k] ? a.we32[j] : 0.f;
+            wl[k] = in[k] && gx > 0 ? a.we32[j - 1] : 0.f;
+            wn[k + 1] = in[k] ? a.wn32[j] : 0.f;
+            dg[k] = in[k] ? a.dg32[j] : 1.f;
+            wd[k] = in[k] ? a.wd32[j] : 0.f;
+        }
+        own = buf + s * FS_H * FS_LD + col;
+        left = own - (col > 0 ? 1 : 0);
+        right = own + (col + 1 < FS_R ? 1 : 0);
+        up = own - (s > 0 ? FS_LD : 0);
+        down = own + ((s + 1) * FS_H < FS_R ? FS_H : FS_H - 1) * FS_LD;
+    }
+    __device__ __forceinline__ void publish(int b) const {
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) own[b * FS_R * FS_LD + k * FS_LD] = u[k];
+    }
+    // r - A u, u being in buffer b
+    __device__ __forceinline__ void residual(int b, float (&res)[FS_H]) const {
+        const int o = b * FS_R * FS_LD;
+        const float top = up[o], bot = down[o];
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) {
+            float v = __fmul_rn(dg[k], u[k]);
+            v = __fmaf_rn(-wl[k], left[o + k * FS_LD], v);
+            v = __fmaf_rn(-we[k], right[o + k * FS_LD], v);
+            v = __fmaf_rn(-wn[k], k > 0 ? u[k > 0 ? k - 1 : 0] : top, v);
+            v = __fmaf_rn(-wn[k + 1], k + 1 < FS_H ? u[k + 1 < FS_H ? k + 1 : k] : bot, v);
+            res[k] = __fsub_rn(r[k], v);
+        }
+    }
+    __device__ __forceinline__ void sweep(int b) {
+        float res[FS_H];
+        residual(b, res);
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) u[k] = __fmaf_rn(wd[k], res[k], u[k]);
+    }
+};
+
+// k_fp_pre at the default depth.  The block after the tiles' does the bookkeeping.
+__global__ void __launch_bounds__(32 * FS_NW, 2) k_fp_pre_strips(FpArgs a, int tick, int net_next) {
+    pdl_enter();
+    FP_MEMBER(a);
+    const int bx = blockIdx.x, t = threadIdx.x;
+    if (bx == a.ntiles2) {
+        fp_pre_state<FS_NW>(a, tick);
+        return;
+    }
+    __shared__ float buf[2 * FS_R * FS_LD];
+    __shared__ float res_tile[FP_TILE * FP_TILE];  // r - A z of the tile's cells
+    __shared__ double sm[32];
+    const bool active = t < FS_ACTIVE;
+    FpStrip c;
+    if (active) {
+        c.load(a, bx, buf, t);
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) c.u[k] = __fmul_rn(c.wd[k], c.r[k]);  // sweep 1, from zero
+    }
+#pragma unroll
+    for (int s = 1; s < FS_H; ++s) {
+        if (active) c.publish(s & 1);
+        __syncthreads();
+        if (active) c.sweep(s & 1);
+    }
+    // the strips of the tile's own cells
+    const int ty = t / FS_R - 1, tx = t % FS_R - FS_H;
+    const bool own = active && ty >= 0 && ty < FP_TILE / FS_H && tx >= 0 && tx < FP_TILE;
+    if (own) {
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k)
+            if (c.in[k]) a.za[c.i + k * c.nx] = (double)c.u[k];
+    }
+    if (!net_next) return;
+    if (active) c.publish(FS_H & 1);
+    __syncthreads();
+    if (own) {
+        float v[FS_H];
+        c.residual(FS_H & 1, v);
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) {
+            if (c.in[k]) a.r1[c.i + k * c.nx] = (double)v[k];
+            res_tile[(ty * FS_H + k) * FP_TILE + tx] = c.in[k] ? v[k] : 0.f;
+        }
+    }
+    __syncthreads();
+    // |r1|^2 in the tile's tree: rows over lanes, then over the 32 rows
+    const int lane = t & 31, warp = t >> 5;
+#pragma unroll
+    for (int row = warp; row < FP_TILE; row += FS_NW) {
+        const double v = (double)res_tile[row * FP_TILE + lane];
+        const double q = warp_xor_sum(__dmul_rn(v, v));
+        if (lane == 0) sm[row] = q;
+    }
+    // restriction of this tile's cells (f divides FP_TILE and the tile origin)
+    const int f = a.f, cs = FP_TILE / f;
+    for (int q = t; q < cs * cs; q += 32 * FS_NW) {
+        const int cx = q % cs, cy = q / cs;
+        const int gx = (bx % a.tx2) * FP_TILE + cx * f, gy = (bx / a.tx2) * FP_TILE + cy * f;
+        if (gx < a.op.nx && gy < a.op.ny) {
+            double sum = 0;
+            for (int dy = 0; dy < f; ++dy)
+                for (int dx = 0; dx < f; ++dx) sum += (double)res_tile[(cy * f + dy) * FP_TILE + cx * f + dx];
+            const int ic = (gy / f) * a.ncx + gx / f;
+            const float m = (float)(sum / (f * f));
+            if (net_next & 2)
+                a.out[ic] = m;
+            else
+                a.xin[2 * ic] = m;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const double q = warp_xor_sum(sm[lane]);
+        if (lane == 0) fslot(a, FP_R1)[bx] = q;
+    }
+}
+
+// k_fp_post at the default depth.
+__global__ void __launch_bounds__(32 * FS_NW, 2) k_fp_post_strips(FpArgs a, int use_y) {
+    pdl_enter();
+    FP_MEMBER(a);
+    const int bx = blockIdx.x, t = threadIdx.x;
+    __shared__ float buf[2 * FS_R * FS_LD];
+    __shared__ double red[64], smm[FP_MAX_TRUNC * FP_TILE];
+    const bool active = t < FS_ACTIVE;
+    const int lane = t & 31, warp = t >> 5;
+    const int x0 = (bx % a.tx2) * FP_TILE, y0 = (bx / a.tx2) * FP_TILE;
+    const int k_it = (int)a.st->k, nj = min(a.m, k_it);
+    FpStrip c;
+    double za[FS_H];
+    float y[FS_H];
+    if (active) {
+        c.load(a, bx, buf, t);
+        const int gx = x0 - FS_H + t % FS_R, gy = y0 - FS_H + t / FS_R * FS_H;
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) {
+            const bool has = use_y && c.in[k] && gx < a.mx && gy + k < a.my;
+            za[k] = c.in[k] ? a.za[c.i + k * c.nx] : 0.0;
+            y[k] = has ? a.out[((gy + k) >> a.fsh) * a.ncx + (gx >> a.fsh)] : 0.f;
+        }
+    }
+    double w = 0.0;  // without the network's y this iteration: smoothing alone
+    if (use_y) {
+        double yr, yay;
+        partial_sums<2, FS_NW>(fslot(a, FP_YR), fslot(a, FP_YAY), a.ntiles, red, &yr, &yay);
+        w = yay > 0 ? yr / yay : 0.0;
+    }
+    if (active) {
+        const int gx = x0 - FS_H + t % FS_R, gy = y0 - FS_H + t / FS_R * FS_H;
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k)
+            c.u[k] = __double2float_rn(w != 0.0 && gx < a.mx && gy + k < a.my ? __fma_rn(w, (double)y[k], za[k])
+                                                                              : za[k]);
+    }
+#pragma unroll
+    for (int s = 0; s < FS_H; ++s) {
+        if (active) c.publish(s & 1);
+        __syncthreads();
+        if (active) c.sweep(s & 1);
+    }
+    const int ty = t / FS_R - 1, tx = t % FS_R - FS_H;
+    const bool own = active && ty >= 0 && ty < FP_TILE / FS_H && tx >= 0 && tx < FP_TILE;
+    float *z = buf + (FS_H & 1) * FS_R * FS_LD;  // the tile's z, rows of FS_LD
+    if (own) {
+#pragma unroll
+        for (int k = 0; k < FS_H; ++k) {
+            if (c.in[k]) {
+                if (a.mixed) a.z32[c.i + k * c.nx] = c.u[k];
+                else a.z[c.i + k * c.nx] = (double)c.u[k];
+            }
+            z[(ty * FS_H + k) * FS_LD + tx] = c.u[k];
+        }
+    }
+    if (nj == 0) return;
+    __syncthreads();
+    // <z, s_{k-1-j}> in the tile's tree: rows over lanes, then over the 32 rows
+#pragma unroll
+    for (int row = warp; row < FP_TILE; row += FS_NW) {
+        const bool in = x0 + lane < a.op.nx && y0 + row < a.op.ny;
+        const int i = (y0 + row) * a.op.nx + x0 + lane;
+        const float zi = z[row * FS_LD + lane];
+#pragma unroll
+        for (int j = 0; j < FP_MAX_TRUNC; ++j) {
+            if (j >= nj) break;
+            const size_t o = (size_t)((k_it - 1 - j) % a.ring) * a.sstride;
+            double v = in ? (a.mixed ? xprod(zi, a.sring32[o + i]) : __dmul_rn((double)zi, a.sring[o + i])) : 0.0;
+            v = warp_xor_sum(v);
+            if (lane == 0) smm[j * FP_TILE + row] = v;
+        }
+    }
+    __syncthreads();
+    if (warp < nj) {
+        const double v = warp_xor_sum(smm[warp * FP_TILE + lane]);
+        if (lane == 0) fslot(a, FP_ZS + warp)[bx] = v;
+    }
 }
 
 size_t fp_smem_bytes(int H) { return 7 * sizeof(float) * (size_t)(FP_TILE + 2 * H) * (FP_TILE + 2 * H); }
@@ -1130,9 +1362,9 @@ __global__ void __launch_bounds__(CG_TILE, 2)
                     case FPP_MSPMV: k_fpm_spmv_blk(a, vb); break;
                     case FPP_MUPDATE: k_fpm_update_blk(a, vb); break;
                     case FPP_MRELIABLE: k_fpm_reliable_blk(a, vb); break;
-                    case FPP_PRE: k_fp_pre_blk<0>(a, vb, ox, oy); break;
+                    case FPP_PRE: k_fp_pre_blk(a, vb, ox, oy); break;
                     case FPP_YDOTS: k_fp_ydots_blk(a, vb); break;
-                    case FPP_POST: k_fp_post_blk<0>(a, vb, ox); break;
+                    case FPP_POST: k_fp_post_blk(a, vb, ox); break;
                     case FPP_DIR: k_fp_dir_blk(a, vb, cond, ox); break;
                     default: break;
                 }
@@ -1373,14 +1605,21 @@ int fp_precond_dir(cfm_fpcg *h, const FpArgs &a, cudaGraphConditionalHandle cond
     cudaStream_t s = h->stream;
     const int net_next = !h->net ? 3 : use_net ? 1 : 0;
     const int M = h->nmem;
-    const auto pre = h->smooth == 4 ? k_fp_pre<4> : k_fp_pre<0>;
-    const auto post = h->smooth == 4 ? k_fp_post<4> : k_fp_post<0>;
     const auto dir = h->m == 1 ? k_fp_dir_spmv : k_fp_dir;
-    CFM_CUDA_TRY(launch_pdl(pre, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(std::max(h->smooth, 1)), s, a,
-                            tick, net_next));
+    // the default depth in registers
+    const bool strips = h->smooth == FS_H;
+    auto post = [&](int use_y) {
+        return strips ? launch_pdl(k_fp_post_strips, dim3(h->ntiles2, M), dim3(32 * FS_NW), 0, s, a, use_y)
+                      : launch_pdl(k_fp_post, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(h->smooth), s, a, use_y);
+    };
+    if (strips)
+        CFM_CUDA_TRY(launch_pdl(k_fp_pre_strips, dim3(h->ntiles2 + 1, M), dim3(32 * FS_NW), 0, s, a, tick, net_next));
+    else
+        CFM_CUDA_TRY(launch_pdl(k_fp_pre, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(std::max(h->smooth, 1)), s,
+                                a, tick, net_next));
     if (!net_next) {
         // smoothing alone this iteration: no r1, no network, c = 0
-        CFM_CUDA_TRY(launch_pdl(post, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(h->smooth), s, a, 0));
+        CFM_CUDA_TRY(post(0));
         CFM_CUDA_TRY(launch_pdl(dir, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a, cond, set_cond));
         return CFM_OK;
     }
@@ -1389,7 +1628,7 @@ int fp_precond_dir(cfm_fpcg *h, const FpArgs &a, cudaGraphConditionalHandle cond
         if (st) return st;
     }
     CFM_CUDA_TRY(launch_pdl(k_fp_ydots, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a));
-    CFM_CUDA_TRY(launch_pdl(post, dim3(h->ntiles2, M), dim3(CG_TILE), fp_smem_bytes(h->smooth), s, a, 1));
+    CFM_CUDA_TRY(post(1));
     CFM_CUDA_TRY(launch_pdl(dir, dim3(h->ntiles, M), dim3(CG_TILE), 0, s, a, cond, set_cond));
     return CFM_OK;
 }
@@ -1566,21 +1805,13 @@ int fp_setup(cfm_fpcg *h, int nx, int ny, int f, cfm_unet *net, int smooth, int 
         (e = cudaMalloc(&h->xin, sizeof(float) * 2 * (size_t)h->nc * nmem)) != cudaSuccess ||
         (e = cudaMalloc(&h->out, sizeof(float) * (size_t)h->nc * nmem)) != cudaSuccess ||
         (e = cudaMalloc(&h->part, sizeof(double) * FP_NSLOT * (size_t)h->pstride * nmem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_pre<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (e = cudaFuncSetAttribute(k_fp_pre, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_pre<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (e = cudaFuncSetAttribute(k_fp_post, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_post<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_post<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)fp_smem_bytes(FP_MAX_SMOOTH))) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_pre<0>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        (e = cudaFuncSetAttribute(k_fp_pre, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_pre<4>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_post<0>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_fp_post<4>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        (e = cudaFuncSetAttribute(k_fp_post, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
         (e = cudaMalloc(&h->acc, sizeof(double) * std::max(4, nmem))) != cudaSuccess ||
         (e = cudaMalloc(&h->rslots, sizeof(double) * FP_RES_BLOCKS * (size_t)nmem)) != cudaSuccess ||

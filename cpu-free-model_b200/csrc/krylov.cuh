@@ -62,23 +62,28 @@ __device__ __forceinline__ double block_sum(double v, double *sm /* 32 doubles *
     return out;
 }
 
-// One or two sums of tile partials in the fixed order (thread t adds part[t],
+// One or two sums of tile partials in the fixed order (thread t of 1024 adds part[t],
 // part[t+1024], ..., then the tree of block_sum) behind one block barrier: every warp
-// adds the 32 warp sums for itself.  sm: N x 32 doubles that no thread still reads.
-template <int N>
+// adds the 32 warp sums for itself.  Blocks of NW < 32 warps take several of the 32 warps'
+// parts per warp.  sm: N x 32 doubles that no thread still reads.
+template <int N, int NW = 32>
 __device__ __forceinline__ void partial_sums(const double *p, const double *p2, int ntiles, double *sm, double *out,
                                              double *out2) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double v = 0.0, v2 = 0.0;
-    for (int i = threadIdx.x; i < ntiles; i += CG_TILE) {
-        v = __dadd_rn(v, p[i]);
-        if (N > 1) v2 = __dadd_rn(v2, p2[i]);
-    }
-    v = warp_xor_sum(v);
-    if (N > 1) v2 = warp_xor_sum(v2);
-    if (lane == 0) {
-        sm[warp] = v;
-        if (N > 1) sm[32 + warp] = v2;
+    static_assert(32 % NW == 0, "whole turns");
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int warp = threadIdx.x >> 5; warp < 32; warp += NW) {
+        double v = 0.0, v2 = 0.0;
+        for (int i = warp * 32 + lane; i < ntiles; i += CG_TILE) {
+            v = __dadd_rn(v, p[i]);
+            if (N > 1) v2 = __dadd_rn(v2, p2[i]);
+        }
+        v = warp_xor_sum(v);
+        if (N > 1) v2 = warp_xor_sum(v2);
+        if (lane == 0) {
+            sm[warp] = v;
+            if (N > 1) sm[32 + warp] = v2;
+        }
     }
     __syncthreads();
     *out = warp_xor_sum(sm[lane]);
