@@ -959,19 +959,26 @@ __global__ void __launch_bounds__(32 * FS_NW, 2) k_fp_post_strips(FpArgs a, int 
     if (nj == 0) return;
     __syncthreads();
     // <z, s_{k-1-j}> in the tile's tree: rows over lanes, then over the 32 rows
-#pragma unroll
+    const int slot = (k_it - 1) % a.ring;
+#pragma unroll 1
     for (int row = warp; row < FP_TILE; row += FS_NW) {
         const bool in = x0 + lane < a.op.nx && y0 + row < a.op.ny;
         const int i = (y0 + row) * a.op.nx + x0 + lane;
         const float zi = z[row * FS_LD + lane];
+        double v[FP_MAX_TRUNC];  // all loads before the first sum
+        int q = slot;
 #pragma unroll
         for (int j = 0; j < FP_MAX_TRUNC; ++j) {
-            if (j >= nj) break;
-            const size_t o = (size_t)((k_it - 1 - j) % a.ring) * a.sstride;
-            double v = in ? (a.mixed ? xprod(zi, a.sring32[o + i]) : __dmul_rn((double)zi, a.sring[o + i])) : 0.0;
-            v = warp_xor_sum(v);
-            if (lane == 0) smm[j * FP_TILE + row] = v;
+            const size_t o = (size_t)q * a.sstride + i;
+            v[j] = j < nj && in ? (a.mixed ? xprod(zi, a.sring32[o]) : __dmul_rn((double)zi, a.sring[o])) : 0.0;
+            q = q > 0 ? q - 1 : a.ring - 1;
         }
+#pragma unroll
+        for (int j = 0; j < FP_MAX_TRUNC; ++j)
+            if (j < nj) {
+                const double w = warp_xor_sum(v[j]);
+                if (lane == 0) smm[j * FP_TILE + row] = w;
+            }
     }
     __syncthreads();
     if (warp < nj) {
@@ -1026,41 +1033,58 @@ __global__ void __launch_bounds__(CG_TILE) k_fp_ydots(FpArgs a) {
 // directions (into ring slot k mod (m + 1)), partial <p_k, r_k>, and the
 // loop condition.
 __device__ __forceinline__ void k_fp_dir_blk(const FpArgs &a, int bx, cudaGraphConditionalHandle cond, int set_cond) {
-    __shared__ double sm[33];
+    __shared__ double sm[33], parts[FP_MAX_TRUNC * 32], beta[FP_MAX_TRUNC];
     const int k = (int)a.st->k;
     const int nj = min(a.m, k);
-    __shared__ const double *pj[FP_MAX_TRUNC];
-    if (threadIdx.x < nj) pj[threadIdx.x] = a.pring + (size_t)((k - 1 - (int)threadIdx.x) % a.ring) * a.sstride;
-    double beta[FP_MAX_TRUNC];
-    if (nj > 0) {
-        __shared__ double smm[33 * FP_MAX_TRUNC];
-#pragma unroll
-        for (int j = 0; j < FP_MAX_TRUNC; ++j) {
-            double acc = 0.0;
-            if (j < nj)
-                for (int t = threadIdx.x; t < a.ntiles2; t += blockDim.x) acc += fslot(a, FP_ZS + j)[t];
-            beta[j] = acc;
-        }
-        block_sum_multi(beta, nj, smm);
-        for (int j = 0; j < nj; ++j) {
-            const double ps = a.st->ps[(k - 1 - j) % a.ring];
-            beta[j] = ps != 0.0 ? beta[j] / ps : 0.0;
-        }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The nj sums in block_sum's tree, their warps' parts shared out over this block's
+    // warps (beyond ntiles2 a warp's part is 0): two barriers for all of them.
+    const int nw = min(32, (a.ntiles2 + 31) / 32);
+    for (int q = warp; q < nj * nw; q += 32) {
+        const int j = q / nw, w = q - j * nw;
+        double acc = 0.0;
+        for (int t = w * 32 + lane; t < a.ntiles2; t += CG_TILE) acc = __dadd_rn(acc, fslot(a, FP_ZS + j)[t]);
+        acc = warp_xor_sum(acc);
+        if (lane == 0) parts[j * 32 + w] = acc;
     }
-    __syncthreads();  // pj
+    __syncthreads();
+    if (warp < nj) {
+        const double zs = warp_xor_sum(lane < nw ? parts[warp * 32 + lane] : 0.0);
+        const double ps = a.st->ps[(k - 1 - warp) % a.ring];
+        if (lane == 0) beta[warp] = ps != 0.0 ? zs / ps : 0.0;
+    }
+    __syncthreads();
     const int i = bx * CG_TILE + threadIdx.x;
     double pr = 0;
     if (i < a.n) {
+        int q = nj > 0 ? (k - 1) % a.ring : 0;  // ring slot of p_{k-1-j}
         if (a.mixed) {  // FP32 direction, beta rounded to FP32
-            float pi = a.z32[i];
-            for (int j = 0; j < nj; ++j)
-                pi = __fmaf_rn(-__double2float_rn(beta[j]),
-                               a.pring32[(size_t)((k - 1 - j) % a.ring) * a.sstride + i], pi);
+            float pi = a.z32[i], v[FP_MAX_TRUNC];
+#pragma unroll
+            for (int j = 0; j < FP_MAX_TRUNC; ++j) {
+                v[j] = j < nj ? a.pring32[(size_t)q * a.sstride + i] : 0.f;
+                q = q > 0 ? q - 1 : a.ring - 1;
+            }
+#pragma unroll
+            for (int j = 0; j < FP_MAX_TRUNC; ++j)
+                if (j < nj) pi = __fmaf_rn(-__double2float_rn(beta[j]), v[j], pi);
             a.pring32[(size_t)(k % a.ring) * a.sstride + i] = pi;
             pr = xprod(pi, a.r32[i]);
         } else {
             double pi = a.z[i];
-            for (int j = 0; j < nj; ++j) pi = __fma_rn(-beta[j], pj[j][i], pi);
+            constexpr int G = 4;  // loads ahead
+#pragma unroll
+            for (int j0 = 0; j0 < FP_MAX_TRUNC; j0 += G) {
+                double v[G];
+#pragma unroll
+                for (int j = 0; j < G; ++j) {
+                    v[j] = j0 + j < nj ? a.pring[(size_t)q * a.sstride + i] : 0.0;
+                    q = q > 0 ? q - 1 : a.ring - 1;
+                }
+#pragma unroll
+                for (int j = 0; j < G; ++j)
+                    if (j0 + j < nj) pi = __fma_rn(-beta[j0 + j], v[j], pi);
+            }
             a.pring[(size_t)(k % a.ring) * a.sstride + i] = pi;
             pr = __dmul_rn(pi, a.r[i]);
         }
@@ -1070,7 +1094,7 @@ __device__ __forceinline__ void k_fp_dir_blk(const FpArgs &a, int bx, cudaGraphC
     if (set_cond && bx == 0 && threadIdx.x == 0)
         cudaGraphSetConditional(cond, a.st->done ? 0u : 1u);
 }
-__global__ void __launch_bounds__(CG_TILE) k_fp_dir(FpArgs a, cudaGraphConditionalHandle cond, int set_cond) {
+__global__ void __launch_bounds__(CG_TILE, 2) k_fp_dir(FpArgs a, cudaGraphConditionalHandle cond, int set_cond) {
     pdl_enter();
     FP_MEMBER(a);
     k_fp_dir_blk(a, blockIdx.x, cond, set_cond);
