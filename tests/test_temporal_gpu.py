@@ -160,3 +160,20 @@ def test_batch_starting_plan_covers_every_system():
         assert (it0 == it1).all() and (st0 == st1).all()
         for i in range(B.n):
             np.testing.assert_array_equal(B.solution(i), xs[i])
+
+
+# One tile, one tile and a remainder of two cells each way, fewer rows than a strip's four
+# plus its halo, a remainder of half a tile in x.
+@pytest.mark.parametrize("shape", [(32, 32), (34, 66), (6, 70), (68, 48)])
+@pytest.mark.parametrize("m", [1, 3])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_fpcg_smoothing_in_registers(shape, m, mixed):
+    ny, nx = shape
+    k, f = cfm.varcoef_problem(shape, 45)
+    want, its, _, done = oracle.fpcg2d((nx, ny), cfm.varcoef_coeffs(k), f, 4, m, mixed)
+    assert done == 1
+    fp = cfm.FPCG(cfm.Stencil(k), k, None, maxiter=20000, tol=1e-8, smooth=4, truncation=m,
+                  precision=cfm.FP32 if mixed else None)
+    x, st = fp.solve(f)
+    assert st.status == cfm.OK and st.iterations == its
+    np.testing.assert_array_equal(x, want)
