@@ -11,8 +11,10 @@ from the previous grid, which does not change the work.  Metric: GLUP/s
          around K steps (each step = edge preset + one cooperative launch).
   e2e    the same metric through the C ABI with pinned host buffers:
          cfm_jacobi_run_host = H2D of the grid, the sweeps, D2H of the result.
-  roofline  16 algorithmic bytes per LUP over the measured launch time,
-         against MEASURED_PEAKS.json's copy bandwidth.
+  roofline  the bytes of the passes over the grid (16 per interior point and
+         pass; a shape with two sweeps per pass makes about half as many
+         passes as sweeps) over the measured launch time, against
+         MEASURED_PEAKS.json's copy bandwidth.
   cpu_baseline  the oracle's FP64 sweep loop (C/OpenMP) on the host cores.
 
   secondary  (one GPU, after the timed regions; --no-secondary skips it) the
@@ -878,7 +880,10 @@ def main():
     e2e_value = whole_job_rate(world, e2e_steps, lup_step, e2e_s) / 1e9
     peak, peak_kind = peak_hbm()
     per_launch_s = kern_s / args.steps
-    achieved = BYTES_PER_LUP * lup_step / per_launch_s / 1e9
+    # passes over the grid per step: the first sweep alone, then tuned[3] sweeps each
+    passes = NITER if tuned is None or tuned[3] == 1 else 1 + NITER // 2
+    pass_bytes = BYTES_PER_LUP * LUP_PER_SWEEP * passes
+    achieved = pass_bytes / per_launch_s / 1e9
     traffic = traffic_per_launch()
     line = {
         "metric": "Jacobi 3d7p 512^3 FP64 GLUP/s", "value": value, "unit": "GLUP/s", "n_gpus": world,
@@ -887,7 +892,7 @@ def main():
         "data": "synthetic",
         "config": {"workload": "jacobi3d7p_512^3_fp64_periodic", "nx": N, "ny": N, "nz": N,
                    "niter_per_step": NITER, "problem": "config (x faces sin*sin, periodic y,z)",
-                   "impl": "persistent cooperative kernel, grid barrier per sweep",
+                   "impl": "persistent cooperative kernel, grid barrier per pass",
                    "launch": f"{blocks}x{threads}", "parallelism": f"replicas x{world}",
                    "tuned": None if tuned is None else
                    {"variant": best, "consumer_warps": tuned[0], "rows_per_warp": tuned[1], "stages": tuned[2],
@@ -895,7 +900,7 @@ def main():
                    "l2": "inputs larger than L2 (two 1.07 GB grids)"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic,
-                     "algorithmic_bytes_per_launch": BYTES_PER_LUP * lup_step},
+                     "passes_per_launch": passes, "algorithmic_bytes_per_launch": pass_bytes},
         "clocks": clk,
         "e2e": {"value": e2e_value, "unit": "GLUP/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "steps": e2e_steps,
