@@ -10,8 +10,8 @@
 // the neighbouring tiles.  A producer warp copies the planes of the unit, one after the
 // other, into a ring of S shared-memory stages: one tensor copy (TMA) per plane, or
 // cp.async row by row where the window wraps around in y or the rows are not a multiple
-// of 16 bytes (one warp issues a row in about 57 cycles, which bounded the kernel while
-// every plane came that way: 512^3 FP64 30.4 ms per 100 sweeps); rows and planes wrap as
+// of 16 bytes (512^3 FP64, 100 sweeps: 30.4 ms with every plane by cp.async, 29.1 with the
+// tensor copies); rows and planes wrap as
 // the periodic images do, so the halo planes (and rows, with PY) are read only by the
 // single sweeps.  Consumer warps march along z with everything they own in
 // registers: as plane s arrives, sweep 1 makes plane s - 1 from the planes s - 2,
@@ -21,6 +21,14 @@
 // the ring for sweep 1, and for sweep 2 from a small exchange in shared memory,
 // published one step before it is read, with waits on the two adjacent warps
 // only.
+//
+// 512^3, 100 sweeps on B200, the best one-sweep shape against this: FP64 36.8 to 41 ms, now
+// 27.8 (477 GLUP/s, 3.9 TB/s: 0.59 of a 6.65 TB/s copy); FP32 20.6, now 17.4 (761 GLUP/s).
+// What bounds it now is the consumers' latency: eight warps, two per scheduler, at 1.6
+// instructions per clock and SM, waiting on fixed latencies and shared memory.  168
+// registers per thread (three warps to one scheduler) leave no room for more warps of this
+// shape; two blocks per SM at 96 registers spill or overlap too much (8 x 2 rows 33.1 ms,
+// 8 x 3 38.5, 8 x 4 61.8).
 //
 // Overlap cells are computed from the same inputs by the same operations as by
 // their owners, so the grid is the one-sweep grid bit for bit

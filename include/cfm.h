@@ -150,7 +150,8 @@ int cfm_jacobi_set_boundary(cfm_jacobi *h, int boundary);
  * every sweep, the reference's cg::sync(grid) order
  * (Stencil/jacobi3D/src/single-stream/multi-threaded-two-block-comm.cu:122).
  * Both give the same grid bit for bit; at 512^3 FP64 the barrier order
- * measured 3% faster. */
+ * measured 3% faster at one sweep per pass.  A handle whose shape takes two
+ * sweeps per pass runs this order on the default one-sweep shape. */
 int cfm_jacobi_set_dataflow(cfm_jacobi *h, int on);
 /* Device-side equivalent of cfm_jacobi_problem_host into the handle's grid. */
 int cfm_jacobi_load_problem(cfm_jacobi *h, int problem);
@@ -179,8 +180,9 @@ int cfm_jacobi_autotune(cfm_jacobi *h, int sweeps, int *best_variant, double *be
 /* Shape of compiled pipeline variant `index` (CFM_BAD_ARG past the last). */
 int cfm_jacobi_variant_info(int index, int *consumer_warps, int *rows_per_warp, int *stages);
 /* Sweeps per pass over the grid of pipeline shape `index`: 1, or 2 for the
- * temporally blocked shapes (an odd sweep count ends with one one-sweep
- * launch); a negative status for an unknown index. */
+ * temporally blocked shapes (the first sweep of a run, and the last of an
+ * odd rest, have a pass to themselves in the same launch); a negative status
+ * for an unknown index. */
 int cfm_jacobi_variant_sweeps(int index);
 /* z-chunk (planes per work unit) the 3D persistent kernel of this handle
  * uses (after cfm_jacobi_autotune: the chosen one). */
@@ -481,7 +483,7 @@ int cfm_fpcg_reliable_updates(const cfm_fpcg *h);
  * phases behind bounded grid barriers (the persistent-kernel idea of the
  * reference's CPU-free CG, CG/src/single-stream/standard.cu:158-299,
  * applied to FPCG).  Both compute the same values bit for bit; on B200 the
- * per-phase kernels measured faster (512^2: 38 against 48 ms for
+ * per-phase kernels measured faster (512^2: 28 against 43 ms for
  * Jacobi-smoothed FPCG).  Batches always use the per-phase kernels. */
 int cfm_fpcg_set_device_loop(cfm_fpcg *h, int on);
 /* A batch of independent 2D variable-coefficient systems solved together
@@ -521,7 +523,9 @@ int cfm_fpcg_history(cfm_fpcg *h, double *out, long long max_n, long long *n_out
  * cfm_batch_set_precision; damped-Jacobi polynomial preconditioner) behind
  * team-local bounded barriers.  System i: dims[i],
  * nx/ny/nz[i] (nz ignored in 2D), cell coefficients k_host[i] and right-hand
- * side b_host[i] (x0 = 0). */
+ * side b_host[i] (x0 = 0).  Classes and teams start from a plan fitted to the
+ * batch's sizes and precision; cfm_batch_set_plan and cfm_batch_autotune
+ * replace it.  No result depends on the plan. */
 typedef struct cfm_batch cfm_batch;
 int cfm_batch_create(int nsys, const int *dims, const int *nx, const int *ny, const int *nz,
                      const double *const *k_host, const double *const *b_host, cfm_batch **out);
@@ -550,8 +554,8 @@ int cfm_batch_set_precision(cfm_batch *h, int precision, int inner_maxiter, doub
  * time of the launch, stats->iterations = the sum of iterations. */
 int cfm_batch_solve(cfm_batch *h, long long *iters, int *status, double *relres, cfm_stats *st);
 int cfm_batch_solution(cfm_batch *h, int i, double *x_host);
-/* Autotuner: times every built-in plan (class thresholds x team sizes) on
- * the real batch and keeps the fastest. */
+/* Autotuner: times every built-in plan (class thresholds x team sizes, and
+ * the starting plan) on the real batch and keeps the fastest. */
 int cfm_batch_autotune(cfm_batch *h, double *best_ms);
 
 /* -------------------------------------------------------------- testing */
