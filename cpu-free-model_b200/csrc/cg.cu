@@ -344,8 +344,11 @@ int plan_resident(cfm_cg *h, const DeviceInfo &di) {
         if (blocks > di.num_sms) continue;
         const size_t smem = sizeof(double) * (h->kind == 2 ? cgr_smem_doubles<2>(T, h->S->nx, h->S->ny)
                                                            : cgr_smem_doubles<3>(T, h->S->nx, h->S->ny));
-        if (smem > di.smem_optin) return CFM_OK;
         const void *fn = h->kind == 2 ? resident_fn<2>(T) : resident_fn<3>(T);
+        cudaFuncAttributes at;
+        CFM_CUDA_TRY(cudaFuncGetAttributes(&at, fn));
+        // the kernel's static shared memory (its barrier's flag) counts against the limit too
+        if (smem + at.sharedSizeBytes > di.smem_optin) return CFM_OK;
         CFM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
         CFM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, CG_TILE, smem));

@@ -62,6 +62,19 @@ def test_cg_system_on_chip(shape, maxiter):
     np.testing.assert_array_equal(x, xo)
 
 
+# Shapes whose dynamic shared memory on chip is exactly a block's 227 KB, which leaves no
+# room for the kernel's static part: two in 2D (six tiles per block), two in 3D (four).
+@pytest.mark.parametrize("shape", [(150, 4159), (215, 4159), (60, 176, 47), (56, 140, 59)])
+def test_cg_on_chip_at_the_shared_memory_limit(shape):
+    k, f = cfm.varcoef_problem(shape, 37)
+    dims = len(shape)
+    grid = (shape[-1], shape[-2], shape[0] if dims == 3 else 1)
+    xo, _, it_o, _, _ = oracle.krylov_stencil(dims, grid, cfm.varcoef_coeffs(k), f, oracle.STD, 12, 0.0)
+    x, st = cfm.CG(cfm.Stencil(k), cfm.CG_PERSISTENT, 12, 0.0).solve(f.ravel())
+    assert st.iterations == it_o
+    np.testing.assert_array_equal(x, xo)
+
+
 def grid_matrix(shape, values):
     """5-point CSR matrix of a grid: constant values (few row classes with equal values),
     or random symmetric ones (few classes of offsets only)."""
