@@ -348,8 +348,11 @@ int plan_resident(cfm_cg *h, const DeviceInfo &di) {
         cudaFuncAttributes at;
         CFM_CUDA_TRY(cudaFuncGetAttributes(&at, fn));
         // the kernel's static shared memory (its barrier's flag) counts against the limit too
-        if (smem + at.sharedSizeBytes > di.smem_optin) return CFM_OK;
-        CFM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const size_t most = di.smem_optin - at.sharedSizeBytes;
+        if (smem > most) return CFM_OK;
+        // The attribute is the function's, not the handle's: all a block can have, since
+        // another handle's smaller system must not lower it under this one's launches.
+        CFM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         int per_sm = 0;
         CFM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, CG_TILE, smem));
         if (per_sm < 1) return CFM_OK;

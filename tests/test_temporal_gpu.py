@@ -75,6 +75,20 @@ def test_cg_on_chip_at_the_shared_memory_limit(shape):
     np.testing.assert_array_equal(x, xo)
 
 
+# Handles of one kernel whose systems need different amounts of shared memory (narrower
+# rows, or thinner planes, need less), the larger one solved after the smaller was created.
+@pytest.mark.parametrize("large,small", [((480, 500), (1000, 240)), ((60, 60, 60), (240, 30, 30))])
+def test_cg_on_chip_handles_side_by_side(large, small):
+    systems = [cfm.varcoef_problem(s, 38) for s in (large, small)]
+    handles = [cfm.CG(cfm.Stencil(k), cfm.CG_PERSISTENT, 12, 0.0) for k, _ in systems]
+    for (k, f), h in zip(systems, handles):
+        grid = (k.shape[-1], k.shape[-2], k.shape[0] if k.ndim == 3 else 1)
+        xo, _, it_o, _, _ = oracle.krylov_stencil(k.ndim, grid, cfm.varcoef_coeffs(k), f, oracle.STD, 12, 0.0)
+        x, st = h.solve(f.ravel())
+        assert st.iterations == it_o
+        np.testing.assert_array_equal(x, xo)
+
+
 def grid_matrix(shape, values):
     """5-point CSR matrix of a grid: constant values (few row classes with equal values),
     or random symmetric ones (few classes of offsets only)."""
