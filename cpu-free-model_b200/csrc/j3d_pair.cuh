@@ -271,6 +271,13 @@ struct J3PairWarp {
     }
 };
 
+// Waits (bounded) until the last copy into each of the `filled` stages has landed: those
+// before `slot` were filled in this turn around the ring, the others in the one before.  A call of
+// its own: inlined, it costs the consumers registers that spill.
+static __device__ __noinline__ void j3p_drain(uint64_t *full, int filled, int slot, unsigned turn, unsigned long long ns) {
+    for (int i = 0; i < filled; ++i) mbar_wait_bounded(full + i, i < slot ? turn : turn ^ 1, ns > DRAIN_NS ? ns : DRAIN_NS);
+}
+
 template <typename T, int CW, int R, int S, bool PY, bool VEC>
 __global__ void __launch_bounds__(32 * (CW + 1), 1)
     j3d_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, T *g0, T *g1,
@@ -336,6 +343,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1)
             const int h = 1 + (int)((long long)(ty + 1) * PR / nty) - ya;
             const int zb = 1 + ch * zchunk, ze = min(PZ + 1, zb + zchunk);
             if (producer) {
+                if (!w.ok) break;  // (alike in all lanes)
                 // window row l is grid row ya - 2 + l; off-grid columns read as 0
                 const bool on = x0 < nx;
                 const size_t pitch = on ? nx : 0;
@@ -344,7 +352,13 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1)
                 const CUtensorMap *map = in == g0 ? &map0 : &map1;
                 for (int s = zb - H; s < ze + H; ++s, w.next()) {
                     const int slot = w.slot;
-                    if (filled >= S) w.wait(&w.empty[slot], w.turn ^ 1);
+                    if (filled >= S) {
+                        w.wait(&w.empty[slot], w.turn ^ 1);
+                        // (landed long ago, unless a consumer ran out of budget and went on)
+                        w.wait(&w.full[slot], w.turn ^ 1);
+                    }
+                    // after a timeout no more copies: a stage may still be in use
+                    if (!(w.ok = __all_sync(J2_FULL, w.ok))) break;
                     filled = min(filled + 1, S);
                     int z = s;
                     if (site > 0) {  // ring of the planes 1 .. nz-2
@@ -415,11 +429,13 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1)
         }
         left -= pair ? 2 : 1;
         if (producer) cp_async_wait_all();
-        if (!grid_barrier(bar, gridDim.x, site)) return;
+        if (!grid_barrier(bar, gridDim.x, site)) break;
         T *t = in;
         in = out;
         out = t;
     }
+    // on an error exit the block keeps its shared memory until no copy into it is in flight
+    if (producer && w.lane == 0 && ld_relaxed_i32(&bar->error)) j3p_drain(w.full, filled, w.slot, w.turn, w.budget);
     // The result's halo cells (nothing above read any after the first sweep): full
     // rows of the planes 0 and nz-1, and with PY the rows 0 and ny-1 of the others.
     const int warps = gridDim.x * (CW + 1);

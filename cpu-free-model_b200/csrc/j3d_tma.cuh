@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(32 * (CW + 1))
                     }
                     fence_proxy_async_shared();  // reads of the slot before its refill
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty[s]);
+                    if (ok && lane == 0) mbar_arrive(&empty[s]);  // (no refill while its copy is in flight)
                     ++k;
                 }
                 int scur = k % STAGES;
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(32 * (CW + 1))
                 }
                 fence_proxy_async_shared();  // reads of the slot before its refill
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[scur]);
+                if (ok && lane == 0) mbar_arrive(&empty[scur]);
                 if (udone) {
                     // the unit's stores, then one consumer barrier: publish
                     // the unit, or leave together if any consumer failed
@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(32 * (CW + 1))
     // shared memory is released (bounded).
     if (warp == CW && lane == 0 && s_err) {
         const unsigned lo = k > (unsigned)STAGES ? k - STAGES : 0u;
-        for (unsigned j = lo; j < k; ++j) mbar_wait_bounded(&full[j % STAGES], (j / STAGES) & 1, budget);
+        const unsigned long long limit = budget > DRAIN_NS ? budget : DRAIN_NS;
+        for (unsigned j = lo; j < k; ++j) mbar_wait_bounded(&full[j % STAGES], (j / STAGES) & 1, limit);
     }
 }
 

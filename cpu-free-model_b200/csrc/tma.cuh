@@ -59,6 +59,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
     return true;
 }
 
+// How long a block that leaves on an error waits for each of its copies still in
+// flight (at least; a wait's own budget may be far shorter than a copy).
+constexpr unsigned long long DRAIN_NS = 1000000000ull;
+
 // Orders this thread's earlier generic-proxy accesses to the CTA's shared
 // memory before later async-proxy (TMA) accesses to it.  A consumer of a
 // TMA-filled ring slot runs it after its last read of the slot and before

@@ -47,6 +47,26 @@ def test_3d_two_sweeps_per_pass(shape, niter, prec, py):
         np.testing.assert_array_equal(j.download(), oracle.jacobi3d(a, niter, py))
 
 
+def test_3d_two_sweeps_timeout_returns_status_and_handle_stays_usable(monkeypatch):
+    """Waits far shorter than a plane's copy: the run ends with a status (every block lets
+    its copies land first) and the handle's next run is right.  One column of 149 units,
+    so on 148 SMs one block works twice as long as the others wait."""
+    monkeypatch.setenv("CFM_J3D_ZCHUNK", "200")
+    nx, ny, nz = 64, 30, 2 + 149 * 200
+    with cfm.Jacobi(3, nx, ny, nz, cfm.FP64, 1, cfm.JACOBI_PERSISTENT) as j, \
+            cfm.Jacobi(3, nx, ny, nz, cfm.FP64, 1, cfm.JACOBI_HOST_LOOP) as want:
+        j.load_problem(cfm.PROBLEM_CONFIG)
+        cfm.set_barrier_timeout_ms(1e-4)
+        try:
+            assert j.run(5, allowed=(cfm.BARRIER_TIMEOUT,)).status == cfm.BARRIER_TIMEOUT
+        finally:
+            cfm.set_barrier_timeout_ms(2000)
+        for h in (j, want):
+            h.load_problem(cfm.PROBLEM_CONFIG)
+            h.run(5)
+        np.testing.assert_array_equal(j.download(), want.download())
+
+
 # One tile in all, one per block, two, three, four and six per block; systems whose rows all
 # have neighbours in other blocks; beyond the chip.
 @pytest.mark.parametrize("shape,maxiter", [((20, 30), 400), ((33, 31), 400), ((300, 200), 60), ((450, 500), 40),
