@@ -390,23 +390,28 @@ const void *solver_fn(int impl) {
     }
 }
 
-// Algorithmic HBM bytes of one iteration: operator data plus the vector
-// passes of the method (8 B per FP64 entry read or written, 4 per FP32).
-double bytes_per_iter(const cfm_cg *h) {
+// HBM bytes of `iters` iterations: the operator data that the passes read plus the vector
+// passes of the method (8 B per FP64 entry read or written, 4 per FP32).  Row classes
+// replace column indices and, by value, the values by a byte per row (their tables stay
+// in L1); a system on chip is read once and its solution written once.
+double solve_bytes(const cfm_cg *h, long long iters) {
     const double n = h->n;
     double op64, op32;
     if (h->kind == 0) {
+        const int classes = h->A->classes;
         const double nnz = (double)h->A->nnz;
-        op64 = 12.0 * nnz + 4.0 * (n + 1);
-        op32 = 8.0 * nnz + 4.0 * (n + 1);
+        const double index = classes == 2 ? n : classes == 1 ? n + 4.0 * (n + 1) : 4.0 * nnz + 4.0 * (n + 1);
+        op64 = index + (classes == 2 ? 0.0 : 8.0 * nnz);
+        op32 = index + (classes == 2 ? 0.0 : 4.0 * nnz);
     } else {
-        op64 = 8.0 * h->kind * n;  // dims face arrays + diagonal
-        op32 = 4.0 * h->kind * n;
+        op64 = 8.0 * (h->kind + 1) * n;  // dims face arrays + diagonal
+        op32 = 4.0 * (h->kind + 1) * n;
     }
+    if (h->res_fn) return op64 + 16.0 * n;
     switch (h->p.impl) {
-        case CFM_CG_PERSISTENT_PIPELINED: return op64 + 96.0 * n;
-        case CFM_CG_MIXED: return op32 + 44.0 * n;
-        default: return op64 + 88.0 * n;
+        case CFM_CG_PERSISTENT_PIPELINED: return iters * (op64 + 96.0 * n);
+        case CFM_CG_MIXED: return iters * (op32 + 44.0 * n);
+        default: return iters * (op64 + 88.0 * n);
     }
 }
 
@@ -462,7 +467,7 @@ int solve_t(cfm_cg *h, const Op &op, const double *b_dev, double *x_dev, cfm_sta
         st->seconds = ms * 1e-3;
         st->iterations = r.iters;
         st->residual = relres;
-        st->bytes = (double)r.iters * bytes_per_iter(h);
+        st->bytes = solve_bytes(h, r.iters);
         st->gbs = st->seconds > 0 ? st->bytes / st->seconds * 1e-9 : 0;
         st->h2d_bytes = h2d;
         st->d2h_bytes = d2h;

@@ -478,6 +478,7 @@ struct cfm_jacobi {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int blocks = 0, threads = 0, zchunk = 0;
     int num_sms = 0;
+    int passes = 0;  // passes over the grid of the last run
     // 2D persistent and resident runs: the grid on chip (j2d_tile_kernel,
     // with its blocks' exchange counters) or several sweeps per pass over it
     // (j2d_stream_kernel)
@@ -1017,10 +1018,11 @@ int launch_j2(cfm_jacobi *h, int niter, int *launches) {
         void *args[] = {&in, &out, (void *)&p.nx, (void *)&p.ny, &n, &pl.tl, &h->flags, &h->bar};
         CFM_CUDA_TRY(launch_cooperative(pl.fn, dim3(pl.blocks), dim3(pl.threads), args, pl.smem, h->stream));
         swaps = (niter - 1 + pl.tl.k - 1) / pl.tl.k + 1;  // exchanges after the first sweep, and the result
+        h->passes = 1;
     } else {
         void *args[] = {&in, &out, (void *)&p.nx, (void *)&p.ny, &n, &h->bar};
         CFM_CUDA_TRY(launch_cooperative(pl.fn, dim3(pl.blocks), dim3(pl.threads), args, pl.smem, h->stream));
-        swaps = j2s_passes(niter, pl.ts);
+        swaps = h->passes = j2s_passes(niter, pl.ts);
     }
     h->cur ^= swaps & 1;
     ++*launches;
@@ -1037,7 +1039,8 @@ int launch_tma(cfm_jacobi *h, const TmaConfig &c, int count, int *launches) {
         void *args[] = {(void *)&c.map[cu], (void *)&c.map[cu ^ 1], &g0, &g1, (void *)&p.nx, (void *)&p.ny,
                         (void *)&p.nz, &n, &zc, &h->bar};
         CFM_CUDA_TRY(launch_cooperative(c.fn, dim3(c.blocks), dim3(c.threads), args, c.smem, h->stream));
-        h->cur ^= j3p_passes(count) & 1;
+        h->passes = j3p_passes(count);
+        h->cur ^= h->passes & 1;
         ++*launches;
         return CFM_OK;
     } else {
@@ -1083,6 +1086,7 @@ int reset_barrier(cfm_jacobi *h) {
 
 // Enqueues the sweeps (no synchronisation).
 int enqueue_sweeps(cfm_jacobi *h, int niter, int *launches) {
+    h->passes = niter;  // unless the launch below takes several sweeps in one
     if (niter == 0) return CFM_OK;
     int st;
     // (the mirror sweep reads the edge cells and writes whole rows, and the 2D
@@ -1121,7 +1125,7 @@ int finish_run(cfm_jacobi *h, int niter, int launches, double extra_h2d, double 
         st->iterations = niter;
         st->lups = lup * niter;
         st->glups = st->seconds > 0 ? st->lups / st->seconds * 1e-9 : 0.0;
-        st->bytes = st->lups * 2.0 * (double)h->esize;
+        st->bytes = lup * h->passes * 2.0 * (double)h->esize;
         st->gbs = st->seconds > 0 ? st->bytes / st->seconds * 1e-9 : 0.0;
         st->h2d_bytes = extra_h2d;
         st->d2h_bytes = extra_d2h;

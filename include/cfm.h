@@ -84,7 +84,9 @@ typedef struct cfm_stats {
     long long iterations; /* sweeps (Jacobi) or CG iterations performed */
     double lups;          /* lattice-point updates (Jacobi) */
     double glups;         /* lups / seconds / 1e9 */
-    double bytes;         /* algorithmic HBM bytes of the solve (16 B/LUP FP64, 8 FP32 for Jacobi) */
+    double bytes;         /* HBM bytes that the solve's passes over its data read and write, each word once
+                             per pass (Jacobi: 16 B per interior point and pass in FP64, 8 in FP32, where a
+                             pass may take several sweeps and a grid or system on chip is one pass) */
     double gbs;           /* bytes / seconds / 1e9 */
     double residual;      /* CG: final FP64 true relative residual ||b-Ax||/||b|| */
     double h2d_bytes;     /* host->device bytes copied inside the call */

@@ -224,3 +224,36 @@ def test_fpcg_smoothing_in_registers(shape, m, mixed):
     x, st = fp.solve(f)
     assert st.status == cfm.OK and st.iterations == its
     np.testing.assert_array_equal(x, want)
+
+
+# stats.bytes counts the passes that the launched kernels make: a grid on chip is read and
+# written once, the streaming kernel takes the first sweep alone and then up to eight per pass,
+# the 3D kernel two, and the one-sweep kernels one.
+@pytest.mark.parametrize("dims,shape,prec,impl,niter,passes", [
+    (2, (200, 300), cfm.FP64, cfm.JACOBI_RESIDENT, 50, 1), (2, (200, 300), cfm.FP64, cfm.JACOBI_HOST_LOOP, 7, 7),
+    (2, (2100, 2304), cfm.FP64, cfm.JACOBI_PERSISTENT, 17, 3), (3, (40, 39, 63), cfm.FP64, cfm.JACOBI_PERSISTENT, 10, 6),
+    (3, (128, 128, 128), cfm.FP64, cfm.JACOBI_PERSISTENT, 10, 10)])
+def test_jacobi_bytes_are_those_of_the_passes(dims, shape, prec, impl, niter, passes):
+    with cfm.Jacobi(dims, shape[-1], shape[-2], shape[0] if dims == 3 else 1, prec, 1, impl) as j:
+        st = j.run(niter)
+        points = np.prod([n - 2 for n in shape])
+        assert st.lups == points * niter
+        assert st.bytes == points * passes * 2 * (8 if prec == cfm.FP64 else 4)
+
+
+@pytest.mark.parametrize("kind,index,value", [("constant", lambda n, nnz: n, 0),
+                                              ("variable", lambda n, nnz: n + 4 * (n + 1), 1),
+                                              ("many", lambda n, nnz: 4 * nnz + 4 * (n + 1), 1)])
+def test_cg_bytes_are_those_of_the_operator_form(kind, index, value):
+    rowptr, col, val = many_offsets_matrix(1301) if kind == "many" else grid_matrix((61, 47), kind)
+    n, nnz = len(rowptr) - 1, len(val)
+    A = cfm.CSR(rowptr, col, val)
+    for impl, word, vectors in ((cfm.CG_PERSISTENT, 8, 88), (cfm.CG_PERSISTENT_PIPELINED, 8, 96), (cfm.CG_MIXED, 4, 44)):
+        st = cfm.CG(A, impl, 2000, 1e-8).solve(cfm.uniform(35, n))[1]
+        assert st.bytes == st.iterations * (index(n, nnz) + value * word * nnz + vectors * n)
+
+
+def test_cg_bytes_of_a_system_on_chip_do_not_grow_with_iterations():
+    k, f = cfm.varcoef_problem((60, 70), 39)
+    st = cfm.CG(cfm.Stencil(k), cfm.CG_PERSISTENT, 400, 1e-8).solve(f.ravel())[1]
+    assert st.iterations > 50 and st.bytes == (3 * 8 + 16) * k.size
