@@ -25,6 +25,7 @@
 
 #include "cfm_internal.h"
 #include "cg_resident.cuh"
+#include "csr_classes.h"
 #include "krylov.cuh"
 
 namespace cfm {
@@ -92,68 +93,13 @@ ClassOp<VALS> class_op(const cfm_csr *A) {
     return ClassOp<VALS>{A->rowptr, A->val, A->val32, A->cls, A->len, A->off, A->tval, A->tval32, A->L};
 }
 
-// Groups the rows of a 0-based CSR matrix into classes of equal column offsets
-// (and values, when val is given): cls[i] per row and one representative row per
-// class.  False as soon as there are more than CLS_MAX classes or a row is longer than
-// CLS_MAXLEN.  A row is compared with its predecessor's class first, then looked up.
-bool classify_rows(int n, const int *rp, const int *col, const double *val, std::vector<unsigned char> &cls,
-                   std::vector<int> &reps) {
-    auto same = [&](int i, int j) {
-        const int m = rp[i + 1] - rp[i];
-        if (rp[j + 1] - rp[j] != m) return false;
-        const int a = rp[i], b = rp[j], d = i - j;
-        for (int k = 0; k < m; ++k)
-            if (col[a + k] - d != col[b + k]) return false;
-        return !val || m == 0 || std::memcmp(val + a, val + b, sizeof(double) * m) == 0;
-    };
-    auto hash = [&](int i) {
-        unsigned long long h = (unsigned long long)(rp[i + 1] - rp[i]) + 1;
-        auto mix = [&](unsigned long long v) { h = (h ^ v) * 0x9E3779B97F4A7C15ull, h ^= h >> 29; };
-        for (int k = rp[i]; k < rp[i + 1]; ++k) {
-            mix((unsigned)(col[k] - i));
-            if (val) {
-                unsigned long long b;
-                std::memcpy(&b, val + k, sizeof(b));
-                mix(b);
-            }
-        }
-        return h;
-    };
-    constexpr int SLOTS = 4 * CLS_MAX;
-    std::vector<int> table(SLOTS, -1);
-    cls.assign(n, 0);
-    reps.clear();
-    int last = -1;
-    for (int i = 0; i < n; ++i) {
-        if (last >= 0 && same(i, reps[last])) {
-            cls[i] = (unsigned char)last;
-            continue;
-        }
-        if (rp[i + 1] - rp[i] > CLS_MAXLEN) return false;
-        int s = (int)(hash(i) % SLOTS);
-        while (table[s] >= 0 && !same(i, reps[table[s]])) s = (s + 1) % SLOTS;
-        if (table[s] < 0) {
-            if ((int)reps.size() == CLS_MAX) return false;
-            table[s] = (int)reps.size();
-            reps.push_back(i);
-        }
-        last = table[s];
-        cls[i] = (unsigned char)last;
-    }
-    return true;
-}
-
 // Finds the matrix's row classes and uploads their tables (A->classes stays 0 when
 // there are too many).
 cudaError_t build_classes(cfm_csr *A, const int *rp, const int *col, const double *val) {
-    std::vector<unsigned char> cls;
-    std::vector<int> reps;
-    int kind = 0;
-    if (classify_rows(A->n, rp, col, val, cls, reps))
-        kind = 2;
-    else if (classify_rows(A->n, rp, col, nullptr, cls, reps))
-        kind = 1;
-    if (!kind) return cudaSuccess;
+    const RowClasses rows = find_row_classes(A->n, rp, col, val);
+    const std::vector<unsigned char> &cls = rows.cls;
+    const std::vector<int> &reps = rows.reps;
+    if (!rows.kind) return cudaSuccess;
     int L = 4;
     for (int r : reps) L = std::max(L, (rp[r + 1] - rp[r] + 3) / 4 * 4);
     const size_t C = reps.size(), N = C * L;
@@ -180,7 +126,7 @@ cudaError_t build_classes(cfm_csr *A, const int *rp, const int *col, const doubl
         (e = cudaMemcpy(A->tval, tv.data(), sizeof(double) * N, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(A->tval32, tv32.data(), sizeof(float) * N, cudaMemcpyHostToDevice)) != cudaSuccess)
         return e;
-    A->classes = kind;
+    A->classes = rows.kind;
     A->L = L;
     return cudaSuccess;
 }
@@ -624,16 +570,16 @@ int cfm_csr_create(int n, long long nnz, const int *rowptr, const int *col, cons
     const int base = rowptr[0];
     CFM_ARG_CHECK(base == 0 || base == 1, "rowptr[0] must be 0 or 1");
     CFM_ARG_CHECK((long long)rowptr[n] - base == nnz, "rowptr[n] - base must equal nnz");
-    std::vector<int> rp(rowptr, rowptr + n + 1), cc;
-    for (int i = 0; i < n; ++i)
-        CFM_ARG_CHECK(rowptr[i + 1] >= rowptr[i], "rowptr must be non-decreasing");
+    const char *fault = csr_fault(n, nnz, rowptr, col, base);
+    CFM_ARG_CHECK(!fault, fault);
+    std::vector<int> rp, cc;  // 0-based copies of 1-based arrays
     if (base) {
-        for (auto &v : rp) v -= 1;
-    }
-    cc.assign(col, col + nnz);
-    for (auto &c : cc) {
-        c -= base;
-        CFM_ARG_CHECK(c >= 0 && c < n, "column index out of range");
+        rp.resize(n + 1);
+        cc.resize(nnz);
+        rebase(rowptr, n + 1LL, base, rp.data());
+        rebase(col, nnz, base, cc.data());
+        rowptr = rp.data();
+        col = cc.data();
     }
     cfm_csr *A = new cfm_csr();
     A->n = n;
@@ -644,9 +590,9 @@ int cfm_csr_create(int n, long long nnz, const int *rowptr, const int *col, cons
         (e = cudaMalloc(&A->col, sizeof(int) * nz1)) != cudaSuccess ||
         (e = cudaMalloc(&A->val, sizeof(double) * nz1)) != cudaSuccess ||
         (e = cudaMalloc(&A->val32, sizeof(float) * nz1)) != cudaSuccess ||
-        (e = cudaMemcpy(A->rowptr, rp.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice)) !=
+        (e = cudaMemcpy(A->rowptr, rowptr, sizeof(int) * (n + 1), cudaMemcpyHostToDevice)) !=
             cudaSuccess ||
-        (nnz && (e = cudaMemcpy(A->col, cc.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice)) !=
+        (nnz && (e = cudaMemcpy(A->col, col, sizeof(int) * nnz, cudaMemcpyHostToDevice)) !=
                     cudaSuccess) ||
         (nnz && (e = cudaMemcpy(A->val, val, sizeof(double) * nnz, cudaMemcpyHostToDevice)) !=
                     cudaSuccess)) {
@@ -662,7 +608,7 @@ int cfm_csr_create(int n, long long nnz, const int *rowptr, const int *col, cons
             return CFM_CUDA_ERROR;
         }
     }
-    if ((e = build_classes(A, rp.data(), cc.data(), val)) != cudaSuccess) {
+    if ((e = build_classes(A, rowptr, col, val)) != cudaSuccess) {
         set_error("csr row classes failed: %s", cudaGetErrorString(e));
         cfm_csr_destroy(A);
         return e == cudaErrorMemoryAllocation ? CFM_OUT_OF_MEMORY : CFM_CUDA_ERROR;

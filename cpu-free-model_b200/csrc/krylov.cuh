@@ -292,7 +292,6 @@ struct CsrOp {
 // instead of its column indices (and values) from L2 or HBM, and its gathers wait
 // for that byte instead of rowptr and col in turn.  Entries are taken in row order,
 // so the sums are CsrOp's bit for bit.  Table rows are L entries (a multiple of 4).
-constexpr int CLS_MAX = 256, CLS_MAXLEN = 32;
 template <bool VALS>
 struct ClassOp {
     static constexpr bool ROW_FIRST = true;
