@@ -143,7 +143,8 @@ __host__ __device__ inline int j2_xbound(const J2Tiling &t, int i, int nx) {
 // the grid buffer of the exchange's parity, the block's counter is released,
 // the (at most eight) neighbours' counters are awaited (bounded), and the rim
 // is read back.  A neighbour can be at most one exchange ahead, and writes the
-// other buffer then.
+// other buffer then.  The counters go on counting from run to run (`base`: exchanges before
+// this run, which all blocks have made), so no run begins with setting them to zero.
 //
 // Bound: FP64 issue (16 operations per warp and row of 128) or FP32 issue while
 // a sweep runs, and per exchange the latency of store - release - acquire -
@@ -155,7 +156,7 @@ constexpr size_t j2_tile_smem() {
 template <typename T, int R, int WARPS, bool MIRROR>
 __global__ void __launch_bounds__(32 * WARPS, 1)
     j2d_tile_kernel(T *in, T *other, int nx, int ny, int niter, J2Tiling tl, unsigned int *flags,
-                    BarrierState *bar) {
+                    unsigned int base, BarrierState *bar) {
     constexpr int V = J2T_V, W = J2T_W, Q = V * sizeof(T) / 16;  // 16-byte pieces per lane
     // edge rows of each warp: [parity][warp][first, last][piece][lane]
     extern __shared__ __align__(16) unsigned char j2t_smem[];
@@ -274,14 +275,14 @@ __global__ void __launch_bounds__(32 * WARPS, 1)
         }
         __syncthreads();
         if (warp == 0) {
-            if (lane == 0) st_release_u32(flags + blockIdx.x, e);
+            if (lane == 0) st_release_u32(flags + blockIdx.x, base + e);
             bool ok = true;
             if (lane < 9) {
                 const int qx = bx + lane % 3 - 1, qy = (by + lane / 3 - 1 + tl.ty) % tl.ty;
                 if (qx >= 0 && qx < tl.tx && lane != 4) {
                     const unsigned int *f = flags + qy * tl.tx + qx;
                     const unsigned long long t0 = global_ns(), budget = bar->timeout_ns;
-                    for (unsigned it = 1; ld_acquire_u32(f) < e; ++it) {
+                    for (unsigned it = 1; (int)(ld_acquire_u32(f) - (base + e)) < 0; ++it) {
                         if ((it & 63) != 0) continue;
                         if (ld_relaxed_i32(&bar->error)) {
                             ok = false;

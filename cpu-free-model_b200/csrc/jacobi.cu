@@ -478,12 +478,15 @@ struct cfm_jacobi {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int blocks = 0, threads = 0, zchunk = 0;
     int num_sms = 0;
-    int passes = 0;  // passes over the grid of the last run
+    int passes = 0;         // passes over the grid of the last run
+    bool tile_run = false;  // it was one of j2d_tile_kernel
     // 2D persistent and resident runs: the grid on chip (j2d_tile_kernel,
     // with its blocks' exchange counters) or several sweeps per pass over it
     // (j2d_stream_kernel)
     cfm::J2Plan j2;
     unsigned int *flags = nullptr;
+    unsigned int exchanges = 0;  // what the counters stand at ...
+    bool flags_set = false;      // ... if they do (not before the first run, or after a failed one)
     // 3D pipelines: the chosen shape, and beside a two-sweep shape the one-sweep
     // shape of the neighbourhood order
     bool tma = false;
@@ -852,7 +855,25 @@ int plan_j2(cfm_jacobi *h) {
         best.blocks = per_sm * h->num_sms;
     }
     h->j2 = best;
+    h->flags_set = false;  // other blocks may have counted so far
     return CFM_OK;
+}
+
+// Whether a run of niter sweeps takes the handle's 2D single-launch plan.  Runs of one or
+// two sweeps gain nothing from keeping the grid on chip or from several sweeps per pass, and
+// some are faster on the row-marching kernel (whole rows): two sweeps of a grid on chip from 6 MB on
+// (us on B200, marching against on chip: 1024^2 FP64 19.3 / 24.4, 1200^2 FP64 21.4 / 27.7, 1500^2
+// FP32 19.4 / 23.4; 768^2 FP64, 4.7 MB, 19.3 / 19.7), and one or two sweeps from HBM, where the
+// streaming kernel's overlap columns are read for nothing (two grids of 1.07 GB each, 16384^2 FP32: 390
+// / 448 and 775 / 892; 8192^2 FP32, 537 MB in two, 105 / 114; 4096^2 FP64, 268 MB in two, 60.3 / 57.3).
+// Resident handles keep to the kernel they are named for.
+bool takes_j2(const cfm_jacobi *h, int niter) {
+    const cfm_jacobi_params &p = h->p;
+    if (!h->j2.fn) return false;
+    if (niter > 2 || h->mirror || ((size_t)p.nx * h->esize) % 16 != 0) return true;
+    const double bytes = (double)h->elems * (double)h->esize;
+    if (h->j2.tile) return p.impl == CFM_JACOBI_RESIDENT || niter < 2 || bytes < 6e6;
+    return bytes < 200e6;
 }
 
 dim3 block_of(const cfm_jacobi_params &p) { return p.dims == 2 ? dim3(256) : dim3(32, J3_TY); }
@@ -1014,10 +1035,16 @@ int launch_j2(cfm_jacobi *h, int niter, int *launches) {
     void *in = h->buf[h->cur], *out = h->buf[h->cur ^ 1];
     int n = niter, swaps;
     if (pl.tile) {
-        CFM_CUDA_TRY(cudaMemsetAsync(h->flags, 0, sizeof(unsigned int) * pl.blocks, h->stream));
-        void *args[] = {&in, &out, (void *)&p.nx, (void *)&p.ny, &n, &pl.tl, &h->flags, &h->bar};
+        if (!h->flags_set) {
+            CFM_CUDA_TRY(cudaMemsetAsync(h->flags, 0, sizeof(unsigned int) * h->num_sms, h->stream));
+            h->exchanges = 0;
+        }
+        h->flags_set = false;  // until the run has ended well (finish_run)
+        void *args[] = {&in, &out, (void *)&p.nx, (void *)&p.ny, &n, &pl.tl, &h->flags, &h->exchanges, &h->bar};
         CFM_CUDA_TRY(launch_cooperative(pl.fn, dim3(pl.blocks), dim3(pl.threads), args, pl.smem, h->stream));
         swaps = (niter - 1 + pl.tl.k - 1) / pl.tl.k + 1;  // exchanges after the first sweep, and the result
+        h->exchanges += swaps - 1;
+        h->tile_run = true;
         h->passes = 1;
     } else {
         void *args[] = {&in, &out, (void *)&p.nx, (void *)&p.ny, &n, &h->bar};
@@ -1062,7 +1089,7 @@ int persistent_tma(cfm_jacobi *h, int niter, int *launches) {
 
 int persistent(cfm_jacobi *h, int niter, int *launches) {
     const cfm_jacobi_params &p = h->p;
-    if (h->j2.fn) return launch_j2(h, niter, launches);
+    if (takes_j2(h, niter)) return launch_j2(h, niter, launches);
     if (h->tma) return persistent_tma(h, niter, launches);
     const void *fn = sweep_fn_any(p, true, h->mirror);
     void *in = h->buf[h->cur], *out = h->buf[h->cur ^ 1];
@@ -1087,11 +1114,12 @@ int reset_barrier(cfm_jacobi *h) {
 // Enqueues the sweeps (no synchronisation).
 int enqueue_sweeps(cfm_jacobi *h, int niter, int *launches) {
     h->passes = niter;  // unless the launch below takes several sweeps in one
+    h->tile_run = false;
     if (niter == 0) return CFM_OK;
     int st;
     // (the mirror sweep reads the edge cells and writes whole rows, and the 2D
     // single-launch kernels write the whole grid: no preset)
-    if (h->p.impl != CFM_JACOBI_HOST_LOOP && !h->mirror && !h->j2.fn) {
+    if (h->p.impl != CFM_JACOBI_HOST_LOOP && !h->mirror && !takes_j2(h, niter)) {
         st = h->p.precision == CFM_FP64 ? launch_edge_preset<double>(h)
                                         : launch_edge_preset<float>(h);
         if (st) return st;
@@ -1116,6 +1144,8 @@ int finish_run(cfm_jacobi *h, int niter, int launches, double extra_h2d, double 
     if (s.error) {
         set_error("grid barrier %d timed out", s.where);
         status = CFM_BARRIER_TIMEOUT;
+    } else if (h->tile_run) {
+        h->flags_set = true;
     }
     if (st) {
         const cfm_jacobi_params &p = h->p;

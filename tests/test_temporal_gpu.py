@@ -32,6 +32,24 @@ def test_2d_several_sweeps_per_pass(shape, niter, prec, mirror):
         np.testing.assert_array_equal(j.download(), want)
 
 
+# Runs of one and two sweeps among longer ones on one handle: on either side of the sizes from
+# which short runs go to the row-marching kernel (that one sets the edge cells in a launch of its
+# own), where the counters of the on-chip kernel go on from run to run.
+@pytest.mark.parametrize("shape,prec,impl,marches", [
+    ((700, 1000), cfm.FP64, cfm.JACOBI_PERSISTENT, (0, 0)), ((800, 1000), cfm.FP64, cfm.JACOBI_PERSISTENT, (0, 1)),
+    ((800, 1000), cfm.FP64, cfm.JACOBI_RESIDENT, (0, 0)), ((800, 1001), cfm.FP64, cfm.JACOBI_PERSISTENT, (0, 0)),
+    ((1300, 1160), cfm.FP32, cfm.JACOBI_PERSISTENT, (0, 1)), ((4900, 5000), cfm.FP64, cfm.JACOBI_PERSISTENT, (0, 0)),
+    ((5100, 5000), cfm.FP64, cfm.JACOBI_PERSISTENT, (1, 1)), ((5100, 5000), cfm.FP64, cfm.JACOBI_RESIDENT, (1, 1))])
+def test_2d_short_runs(shape, prec, impl, marches):
+    a = rand_grid(shape, prec, 46)
+    with cfm.Jacobi(2, shape[1], shape[0], 1, prec, 1, impl) as j:
+        j.upload(a)
+        counts = (2, 1, 9, 1, 2, 5, 2)
+        for n in counts:
+            assert j.run(n).launches == (1 + marches[n - 1] if n <= 2 else 1)
+        np.testing.assert_array_equal(j.download(), oracle.jacobi2d(a, sum(counts)))
+
+
 # Rows and columns at the tile edges (rows of a multiple of 16 bytes or not), z chunks that
 # end beside the periodic planes, odd and even counts.
 @pytest.mark.parametrize("py", [0, 1])
