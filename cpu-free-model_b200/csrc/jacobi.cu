@@ -490,6 +490,7 @@ struct cfm_jacobi {
     // 3D pipelines: the chosen shape, and beside a two-sweep shape the one-sweep
     // shape of the neighbourhood order
     bool tma = false;
+    bool tuned = false;  // by the autotuner or the environment, not the default rule
     cfm::TmaConfig tc, tail;
     size_t smem_optin = 0;
     // 2D: the mirror x boundary of the reference's PERKS comparator
@@ -697,19 +698,25 @@ int setup_tma(cfm_jacobi *h, int var, int zchunk = 0) {
     return CFM_OK;
 }
 
-// Two sweeps per pass (shape 12) where the two grids are beyond L2, or so small that the
+// Two sweeps per pass (shape 12) where the two grids are well beyond L2, or so small that the
 // passes' latency and barriers are most of a sweep; between, one sweep per pass (shape
-// 0), which has no overlap to compute twice and runs from L2.  100 sweeps on B200, two
-// against one: 512^3 FP64 29.1 / 41 ms, 256^3 FP64 (268 MB) 5.2 / 5.1, 256^3 FP32 (134 MB) 3.8
-// / 3.25, 192^3 FP64 (113 MB) 2.5 / 2.3, 128^3 FP64 (34 MB) 1.06 / 0.86, 128^3 FP32 (17 MB) 0.66
-// / 0.82, 64^3 FP64 0.46 / 0.77.  Rows that are not a multiple of 16 bytes have no
-// one-sweep shape.  CFM_J3D_TMA_VARIANT (an index into the table) overrides.
-int default_tma_variant(const cfm_jacobi *h) {
+// 0), which has no overlap to compute twice and runs from L2.  100 sweeps on B200, ms, one
+// sweep per pass against two.  FP64: 64^3 0.77 / 0.46, 128^3 (34 MB) 0.86 / 1.06, 192^3 (113 MB) 2.30
+// / 2.61, 224^3 (180 MB) 3.74 / 3.64, 250 x 250 x 256 (256 MB) 4.81 / 4.73, 256^3 (268 MB) 5.26 / 5.42,
+// 264^3 (294 MB) 5.71 / 5.59, 288^3 (382 MB) 7.38 / 5.73, 384^3 18.1 / 12.6, 512^3 41.4 / 27.7.  FP32: 128^3
+// (17 MB) 0.82 / 0.66, 256^3 (134 MB) 3.19 / 4.33, 304^3 (225 MB) 4.72 / 4.85, 320^3 (262 MB) 6.04 / 5.41,
+// 400^3 (512 MB) 12.2 / 12.6, 512^3 23.5 / 17.5.  So between 180 and 330 MB they are within 4% of one
+// another in FP64, and where the tiles' last column hangs over the grid (400^3) beyond it; the line lies
+// where FP32 gains 10%.  Rows that are not a multiple of 16 bytes have no one-sweep shape.
+// CFM_J3D_TMA_VARIANT (an index into the table) overrides.
+int default_tma_variant(cfm_jacobi *h) {
     int n = 0;
     tma_variants(&n);
+    h->tuned = false;
     if (const char *e = std::getenv("CFM_J3D_TMA_VARIANT")) {
         const int v = std::atoi(e);
-        if (v >= 0 && v < n) return v;
+        h->tuned = v >= 0 && v < n;
+        if (h->tuned) return v;
     }
     const double bytes = 2.0 * (double)h->elems * (double)h->esize;
     const bool whole = ((size_t)h->p.nx * h->esize) % 16 == 0;
@@ -1082,9 +1089,28 @@ int launch_tma(cfm_jacobi *h, const TmaConfig &c, int count, int *launches) {
     return CFM_OK;
 }
 
+// The pipeline shape of a run of niter sweeps.  Beside a two-sweep shape of the default
+// rule, short runs of grids that are not far beyond L2 take the one-sweep shape: the first
+// sweep and an odd rest have a pass to themselves, which the two-sweep kernel makes slower
+// (one sweep per pass against two, us on B200: one and two sweeps of 256^3 FP64 (268 MB) 64 / 80 and 120
+// / 172, 320^3 FP64 (524 MB) 119 / 114 and 226 / 261, 384^3 FP64 (906 MB) 193 / 179 and 377 / 378,
+// 100^3 FP64 (16 MB) 18 / 21 and 26 / 31, 64^3 FP64 (4 MB) 18 / 16 and 25 / 22; eight sweeps of 256^3
+// FP64 452 / 496, 272^3 FP64 (322 MB) 480 / 528, 288^3 FP64 (382 MB) 599 / 506, 100 sweeps of those 5.3 /
+// 5.4, 5.9 / 5.9 and 7.4 / 5.7 ms; in FP32 beyond 250 MB neither is ahead throughout: two sweeps of
+// 320^3 137 / 149, of 360^3 190 / 170).
+const TmaConfig &tma_shape(const cfm_jacobi *h, int niter) {
+    if (h->tc.sweeps == 1 || !h->tail.ok) return h->tc;
+    if (h->dataflow) return h->tail;
+    if (h->tuned) return h->tc;
+    const double bytes = 2.0 * (double)h->elems * (double)h->esize;
+    const bool fp64 = h->p.precision == CFM_FP64;
+    const bool few = niter <= 2 ? bytes >= 10e6 && bytes < (fp64 ? 600e6 : 250e6)
+                                : fp64 && niter < 10 && bytes >= 250e6 && bytes < 350e6;
+    return few ? h->tail : h->tc;
+}
+
 int persistent_tma(cfm_jacobi *h, int niter, int *launches) {
-    const bool one = h->dataflow && h->tc.sweeps == 2 && h->tail.ok;
-    return launch_tma(h, one ? h->tail : h->tc, niter, launches);
+    return launch_tma(h, tma_shape(h, niter), niter, launches);
 }
 
 int persistent(cfm_jacobi *h, int niter, int *launches) {
@@ -1435,6 +1461,7 @@ int cfm_jacobi_autotune(cfm_jacobi *h, int sweeps, int *best_variant, double *be
     int n = 0, best = -1, best_zc = 0;
     double best_rate = 0.0;
     tma_variants(&n);
+    h->tuned = true;
     const int zcands[] = {0, 16, 24, 32, 48, 64, 128};  // 0: the cost-model choice
     for (int v = 0; v < n && e == cudaSuccess && st == CFM_OK; ++v) {
         for (int zc : zcands) {

@@ -65,6 +65,22 @@ def test_3d_two_sweeps_per_pass(shape, niter, prec, py):
         np.testing.assert_array_equal(j.download(), oracle.jacobi3d(a, niter, py))
 
 
+# Short runs among longer ones on one handle, which take the one-sweep kernel by the sizes:
+# passes of runs of 1, 2, 4 and 12 sweeps (the two-sweep kernel makes 1, 2, 3 and 7).
+@pytest.mark.parametrize("shape,prec,passes", [
+    ((40, 40, 40), cfm.FP64, (1, 2, 3, 7)), ((90, 100, 100), cfm.FP64, (1, 2, 3, 7)), ((250, 256, 256), cfm.FP64, (1, 2, 4, 7)),
+    ((350, 256, 256), cfm.FP64, (1, 2, 3, 7)), ((250, 512, 256), cfm.FP32, (1, 2, 3, 7))])
+def test_3d_short_runs(shape, prec, passes):
+    a = rand_grid(shape, prec, 47)
+    nz, ny, nx = shape
+    with cfm.Jacobi(3, nx, ny, nz, prec, 1, cfm.JACOBI_PERSISTENT) as j:
+        j.upload(a)
+        points = np.prod([n - 2 for n in shape])
+        for n, want in ((2, passes[1]), (1, passes[0]), (4, passes[2]), (12, passes[3]), (2, passes[1])):
+            assert j.run(n).bytes == points * want * 2 * (8 if prec == cfm.FP64 else 4)
+        np.testing.assert_array_equal(j.download(), oracle.jacobi3d(a, 21, 1))
+
+
 def test_3d_two_sweeps_timeout_returns_status_and_handle_stays_usable(monkeypatch):
     """Waits far shorter than a plane's copy: the run ends with a status (every block lets
     its copies land first) and the handle's next run is right.  One column of 149 units,
