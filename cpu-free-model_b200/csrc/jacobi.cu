@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
@@ -1427,7 +1428,7 @@ int cfm_jacobi_variant_info(int index, int *consumer_warps, int *rows_per_warp, 
 
 int cfm_jacobi_zchunk(cfm_jacobi *h) {
     if (!h) return CFM_BAD_ARG;
-    return h->tma ? h->tc.zchunk : h->zchunk;
+    return h->tma ? tma_shape(h, INT_MAX).zchunk : h->zchunk;
 }
 
 int cfm_jacobi_variant_sweeps(int index) {
@@ -1507,8 +1508,9 @@ int cfm_jacobi_launch_shape(cfm_jacobi *h, int *blocks, int *threads) {
         b = h->j2.blocks;
         t = h->j2.threads;
     } else if (h->tma) {
-        b = h->tc.blocks;
-        t = h->tc.threads;
+        const TmaConfig &c = tma_shape(h, INT_MAX);
+        b = c.blocks;
+        t = c.threads;
     }
     if (blocks) *blocks = b;
     if (threads) *threads = t;

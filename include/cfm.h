@@ -153,7 +153,9 @@ int cfm_jacobi_set_boundary(cfm_jacobi *h, int boundary);
  * (Stencil/jacobi3D/src/single-stream/multi-threaded-two-block-comm.cu:122).
  * Both give the same grid bit for bit; at 512^3 FP64 the barrier order
  * measured 3% faster at one sweep per pass.  A handle whose shape takes two
- * sweeps per pass runs this order on the default one-sweep shape. */
+ * sweeps per pass runs this order on the default one-sweep shape.  Rows that
+ * are not a multiple of 16 bytes have no such shape: there the order stays
+ * that of the grid barrier. */
 int cfm_jacobi_set_dataflow(cfm_jacobi *h, int on);
 /* Device-side equivalent of cfm_jacobi_problem_host into the handle's grid. */
 int cfm_jacobi_load_problem(cfm_jacobi *h, int problem);
@@ -170,7 +172,8 @@ int cfm_jacobi_run_host(cfm_jacobi *h, int niter, const void *host_in, void *hos
                         cfm_stats *st);
 /* Device pointer of the current grid (valid until the next run/destroy). */
 void *cfm_jacobi_device_grid(cfm_jacobi *h);
-/* Blocks and threads the persistent kernels launch with on this device. */
+/* Blocks and threads the persistent kernels launch with on this device
+ * (runs of a few sweeps may take another kernel). */
 int cfm_jacobi_launch_shape(cfm_jacobi *h, int *blocks, int *threads);
 /* Autotuner for the 3D TMA pipeline: times every compiled pipeline shape for
  * `sweeps` sweeps on a saved copy of the current grid, keeps the fastest for

@@ -81,6 +81,21 @@ def test_3d_short_runs(shape, prec, passes):
         np.testing.assert_array_equal(j.download(), oracle.jacobi3d(a, 21, 1))
 
 
+def test_3d_launch_shape_is_that_of_the_sweep_order(monkeypatch):
+    """Neighbourhood order runs on the one-sweep shape; rows that are not a multiple of 16
+    bytes keep the two-sweep kernel."""
+    def shape(nx):
+        with cfm.Jacobi(3, nx, 40, 40, cfm.FP64, 1, cfm.JACOBI_PERSISTENT) as j:
+            barrier = j.launch_shape(), cfm.lib.cfm_jacobi_zchunk(j.h)
+            j.set_dataflow(True)
+            return barrier, (j.launch_shape(), cfm.lib.cfm_jacobi_zchunk(j.h))
+    two, order = shape(64)
+    ragged = shape(63)
+    monkeypatch.setenv("CFM_J3D_TMA_VARIANT", "0")
+    one, _ = shape(64)
+    assert order == one and order != two and ragged[0] == ragged[1]
+
+
 def test_3d_two_sweeps_timeout_returns_status_and_handle_stays_usable(monkeypatch):
     """Waits far shorter than a plane's copy: the run ends with a status (every block lets
     its copies land first) and the handle's next run is right.  One column of 149 units,
