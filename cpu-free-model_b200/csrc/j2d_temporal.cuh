@@ -336,9 +336,12 @@ __global__ void __launch_bounds__(32 * WARPS, 1)
 // are the cell's additions and multiplications.
 constexpr int J2S_D = 8;        // rows in flight per warp (a power of two)
 constexpr int J2S_WARPS = 4;    // warps per block
-// Sweeps per pass: 16384^2 in us per sweep on B200 (one sweep per pass: 394 FP32, 797 FP64),
-// FP32 with four columns per lane 127 / 89 / 91 for 4 / 6 / 8, FP64 with four columns 304 /
-// 262 for 4 / 6 (more do not fit the registers), with two columns 194 for 8.
+// Sweeps per pass.  Eight: 16384^2 FP32 91 us per sweep in long runs (one per pass 394, four 127,
+// twelve 157), FP64 194 (one per pass 797).  Six is 1 to 10% faster in long FP32 runs (100 sweeps in us, six
+// against eight: 2048^2 334 / 367, 4096^2 739 / 786, 8192^2 2411 / 2471, 16384^2 8422 / 8625, mirror boundary
+// alike) and leaves more rest passes in short ones (9 sweeps are two passes with eight, three with six);
+// in FP64, two columns per lane, it is slower from 16384^2 on (20104 / 18347; 4096^2 1281 / 1272).  FP64 with
+// four columns per lane takes at most six (262 us per sweep at 16384^2; more do not fit the registers).
 constexpr int J2S_SWEEPS = 8;
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool on) {
