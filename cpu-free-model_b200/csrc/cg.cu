@@ -269,7 +269,7 @@ int true_relres(cfm_cg *h, const KArgs<Op> &a, double bnorm, double *out) {
     return CFM_OK;
 }
 
-// cg_std_res_kernel for T tiles per block.
+// cg_std_res_kernel for T tiles per block (six only in 2D: in 3D they do not fit).
 template <int D>
 const void *resident_fn(int T) {
     switch (T) {
@@ -277,12 +277,16 @@ const void *resident_fn(int T) {
         case 2: return (const void *)cg_std_res_kernel<D, 2>;
         case 3: return (const void *)cg_std_res_kernel<D, 3>;
         case 4: return (const void *)cg_std_res_kernel<D, 4>;
-        default: return (const void *)cg_std_res_kernel<D, 6>;
+        default: return D == 2 ? (const void *)cg_std_res_kernel<2, 6> : nullptr;
     }
 }
 
 // Standard CG on a stencil runs on chip when one block per SM holds the whole
-// system: the fewest tiles per block that do, up to the shared memory.
+// system: the fewest tiles per block that do, up to the shared memory.  Against
+// cg_std_kernel on B200, us per iteration, by tiles per block.  2D: one (389^2) 6.5 / 9.3, two (512^2) 7.6 /
+// 10.7, three (650^2) 8.9 / 12.9, four (770^2) 10.4 / 14.4, six (930^2) 15.6 / 17.7.  3D: one (53^3) 7.2 / 9.6,
+// two (64^3) 8.9 / 11.4, three (75^3) 11.1 / 14.2, four (83^3) 14.1 / 15.8.  From three tiles on the kernel spills
+// a little (2D six 264 bytes) and is ahead all the same.
 int plan_resident(cfm_cg *h, const DeviceInfo &di) {
     if (h->p.impl != CFM_CG_PERSISTENT || h->kind == 0) return CFM_OK;
     for (int T : {1, 2, 3, 4, 6}) {
@@ -291,6 +295,7 @@ int plan_resident(cfm_cg *h, const DeviceInfo &di) {
         const size_t smem = sizeof(double) * (h->kind == 2 ? cgr_smem_doubles<2>(T, h->S->nx, h->S->ny)
                                                            : cgr_smem_doubles<3>(T, h->S->nx, h->S->ny));
         const void *fn = h->kind == 2 ? resident_fn<2>(T) : resident_fn<3>(T);
+        if (!fn) return CFM_OK;
         cudaFuncAttributes at;
         CFM_CUDA_TRY(cudaFuncGetAttributes(&at, fn));
         // the kernel's static shared memory (its barrier's flag) counts against the limit too

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(CG_TILE, 1)
         }
         if (use_tol && sqrt(gamma1) <= target) {
             // the FP64 true residual decides: t = b - A x from x in global memory
-                double tr[T], q2[T];
+            double tr[T], q2[T];
 #pragma unroll
             for (int t = 0; t < T; ++t)
                 if (nb[t]) a.x[lo + t * CG_TILE + (int)threadIdx.x] = x[t];

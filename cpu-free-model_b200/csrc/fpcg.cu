@@ -1377,21 +1377,19 @@ __global__ void __launch_bounds__(CG_TILE, 2)
     k_fp_loop(const FpArgs a, const FpProgram pg, BarrierState *bar, cudaGraphConditionalHandle cond) {
     for (int s = 0; s < pg.n; ++s) {
         const int code = pg.op[s].code, ox = pg.op[s].x, oy = pg.op[s].y;
-        {
-            const int nvb = (code == FPP_PRE || code == FPP_POST) ? a.ntiles2 : a.ntiles;
-            for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-                switch (code) {
-                    case FPP_SPMV: k_fp_spmv_blk(a, vb); break;
-                    case FPP_UPDATE: k_fp_update_blk(a, vb); break;
-                    case FPP_MSPMV: k_fpm_spmv_blk(a, vb); break;
-                    case FPP_MUPDATE: k_fpm_update_blk(a, vb); break;
-                    case FPP_MRELIABLE: k_fpm_reliable_blk(a, vb); break;
-                    case FPP_PRE: k_fp_pre_blk(a, vb, ox, oy); break;
-                    case FPP_YDOTS: k_fp_ydots_blk(a, vb); break;
-                    case FPP_POST: k_fp_post_blk(a, vb, ox); break;
-                    case FPP_DIR: k_fp_dir_blk(a, vb, cond, ox); break;
-                    default: break;
-                }
+        const int nvb = (code == FPP_PRE || code == FPP_POST) ? a.ntiles2 : a.ntiles;
+        for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+            switch (code) {
+                case FPP_SPMV: k_fp_spmv_blk(a, vb); break;
+                case FPP_UPDATE: k_fp_update_blk(a, vb); break;
+                case FPP_MSPMV: k_fpm_spmv_blk(a, vb); break;
+                case FPP_MUPDATE: k_fpm_update_blk(a, vb); break;
+                case FPP_MRELIABLE: k_fpm_reliable_blk(a, vb); break;
+                case FPP_PRE: k_fp_pre_blk(a, vb, ox, oy); break;
+                case FPP_YDOTS: k_fp_ydots_blk(a, vb); break;
+                case FPP_POST: k_fp_post_blk(a, vb, ox); break;
+                case FPP_DIR: k_fp_dir_blk(a, vb, cond, ox); break;
+                default: break;
             }
         }
         if (s + 1 < pg.n && !grid_barrier(bar, gridDim.x, s)) return;

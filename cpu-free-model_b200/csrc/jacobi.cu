@@ -1078,13 +1078,12 @@ int launch_tma(cfm_jacobi *h, const TmaConfig &c, int count, int *launches) {
         h->cur ^= h->passes & 1;
         ++*launches;
         return CFM_OK;
-    } else {
-        unsigned int *ud = h->dataflow && count > 1 ? h->udone : nullptr;
-        if (ud) CFM_CUDA_TRY(cudaMemsetAsync(ud, 0, sizeof(unsigned int) * c.units, h->stream));
-        void *args[] = {(void *)&c.map[cu], (void *)&c.map[cu ^ 1], &g0, &g1, (void *)&p.nx, (void *)&p.ny,
-                        (void *)&p.nz, &n, &zc, &h->bar, &ud};
-        CFM_CUDA_TRY(launch_cooperative(c.fn, dim3(c.blocks), dim3(c.threads), args, c.smem, h->stream));
     }
+    unsigned int *ud = h->dataflow && count > 1 ? h->udone : nullptr;
+    if (ud) CFM_CUDA_TRY(cudaMemsetAsync(ud, 0, sizeof(unsigned int) * c.units, h->stream));
+    void *args[] = {(void *)&c.map[cu], (void *)&c.map[cu ^ 1], &g0, &g1, (void *)&p.nx, (void *)&p.ny,
+                    (void *)&p.nz, &n, &zc, &h->bar, &ud};
+    CFM_CUDA_TRY(launch_cooperative(c.fn, dim3(c.blocks), dim3(c.threads), args, c.smem, h->stream));
     h->cur ^= (count & 1);
     ++*launches;
     return CFM_OK;

@@ -6,7 +6,7 @@
 //   StencilOp<D> matrix-free cell-centred -div(k grad u), 5-point (D = 2) or
 //                7-point (D = 3): t = d_i u_i, then one fma(-w, u_nb, t) per
 //                neighbour in the order x-1, x+1, y-1, y+1, z-1, z+1
-// Each operator also applies in FP32 (apply32) from FP32 copies of its
+// Each operator also applies in FP32 (applyN32) from FP32 copies of its
 // coefficients, for the inner solve of the mixed-precision method.
 //
 // Solvers, each one cooperative launch for the whole solve:
@@ -186,12 +186,6 @@ struct CsrOp {
         double acc = 0.0;
         const int j1 = rowptr[i + 1];
         for (int j = rowptr[i]; j < j1; ++j) acc = __fma_rn(val[j], x[col[j]], acc);
-        return acc;
-    }
-    __device__ __forceinline__ float apply32(const float *x, int i) const {
-        float acc = 0.f;
-        const int j1 = rowptr[i + 1];
-        for (int j = rowptr[i]; j < j1; ++j) acc = __fmaf_rn(val32[j], x[col[j]], acc);
         return acc;
     }
     // apply for rows i (if v1) and i2 (if v2), their entries interleaved so

@@ -120,7 +120,7 @@ def test_3d_two_sweeps_timeout_returns_status_and_handle_stays_usable(monkeypatc
 # have neighbours in other blocks; beyond the chip.
 @pytest.mark.parametrize("shape,maxiter", [((20, 30), 400), ((33, 31), 400), ((300, 200), 60), ((450, 500), 40),
                                            ((600, 640), 30), ((760, 700), 30), ((930, 900), 20), ((1100, 1000), 20),
-                                           ((50, 50, 50), 60), ((80, 75, 70), 30), ((100, 100, 90), 20)])
+                                           ((50, 50, 50), 60), ((80, 75, 70), 30), ((83, 83, 83), 20), ((100, 100, 90), 20)])
 def test_cg_system_on_chip(shape, maxiter):
     k, f = cfm.varcoef_problem(shape, 33)
     dims = len(shape)
@@ -220,6 +220,46 @@ def test_cg_row_classes(kind, impl, method, base):
     xo, st_o, it_o, rs_o, _ = oracle.krylov_csr(rowptr, col, val, b, method, 2000, 1e-8)
     A = cfm.CSR(rowptr + base, col + base, val)
     x, st = cfm.CG(A, impl, 2000, 1e-8).solve(b)
+    assert st.status == st_o and st.iterations == it_o and st.refinements == rs_o
+    np.testing.assert_array_equal(x, xo)
+
+
+def class_limit_matrix(kind):
+    """Matrices at the limits of the row classes: 256 kinds of rows and 257 (which only the
+    offsets then group), rows of 32 entries and of 33 (no classes), an empty row."""
+    n = 1300
+    rows = [{i: 2.0} for i in range(n)]
+    if kind.endswith("values"):
+        for i in range(n):
+            rows[i][i] = 2.0 + (i % 256) / 64
+        if kind == "257 values":
+            rows[n - 1][n - 1] = 7.0
+    elif kind.endswith("entries"):
+        for c in range(1, int(kind.split()[0])):
+            rows[0][c] = rows[c][0] = -0.05
+    else:
+        for i in range(n - 1):
+            rows[i][i + 1] = rows[i + 1][i] = -0.5
+        for i in (699, 701):
+            del rows[i][700]
+        rows[700] = {}
+    rowptr = np.cumsum([0] + [len(r) for r in rows]).astype(np.int32)
+    col = np.array([c for r in rows for c in sorted(r)], np.int32)
+    val = np.array([r[c] for r in rows for c in sorted(r)])
+    b = cfm.uniform(48, n)
+    b[700] = 0.0  # the empty row's equation
+    return rowptr, col, val, b
+
+
+@pytest.mark.parametrize("impl,method,maxiter,tol", [(cfm.CG_PERSISTENT, oracle.STD, 15, 0.0),
+                                                     (cfm.CG_DISCRETE, oracle.STD, 15, 0.0),
+                                                     (cfm.CG_PERSISTENT_PIPELINED, oracle.PIPELINED, 15, 0.0),
+                                                     (cfm.CG_MIXED, oracle.MIXED, 2000, 1e-8)])
+@pytest.mark.parametrize("kind", ["256 values", "257 values", "32 entries", "33 entries", "empty row"])
+def test_cg_row_class_limits(kind, impl, method, maxiter, tol):
+    rowptr, col, val, b = class_limit_matrix(kind)
+    xo, st_o, it_o, rs_o, _ = oracle.krylov_csr(rowptr, col, val, b, method, maxiter, tol)
+    x, st = cfm.CG(cfm.CSR(rowptr, col, val), impl, maxiter, tol).solve(b)
     assert st.status == st_o and st.iterations == it_o and st.refinements == rs_o
     np.testing.assert_array_equal(x, xo)
 
