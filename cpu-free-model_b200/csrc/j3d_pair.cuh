@@ -10,8 +10,8 @@
 // the neighbouring tiles.  A producer warp copies the planes of the unit, one after the
 // other, into a ring of S shared-memory stages: one tensor copy (TMA) per plane, or
 // cp.async row by row where the window wraps around in y or the rows are not a multiple
-// of 16 bytes (512^3 FP64, 100 sweeps: 30.4 ms with every plane by cp.async, 29.1 with the
-// tensor copies); rows and planes wrap as
+// of 16 bytes (the first form of this kernel, 512^3 FP64, 100 sweeps: 30.4 ms with every plane by
+// cp.async, 29.1 with the tensor copies); rows and planes wrap as
 // the periodic images do, so the halo planes (and rows, with PY) are read only by the
 // single sweeps.  Consumer warps march along z with everything they own in
 // registers: as plane s arrives, sweep 1 makes plane s - 1 from the planes s - 2,
@@ -23,7 +23,7 @@
 // only.
 //
 // 512^3, 100 sweeps on B200, the best one-sweep shape against this: FP64 36.8 to 41 ms, now
-// 27.8 (477 GLUP/s, 3.9 TB/s: 0.59 of a 6.65 TB/s copy); FP32 20.6, now 17.4 (761 GLUP/s).
+// 26.8 (495 GLUP/s, 4.0 TB/s: 0.62 of the measured copy); FP32 20.6, now 17.3 (767 GLUP/s).
 // What bounds it now is the consumers' latency: eight warps, two per scheduler, at 1.6
 // instructions per clock and SM, waiting on fixed latencies and shared memory.  168
 // registers per thread (three warps to one scheduler) leave no room for more warps of this
@@ -111,18 +111,45 @@ struct J3PairWarp {
     int slot, prev;  // ring stages of the next plane and the one before it
     unsigned turn;   // parity of the turns around the ring so far
     unsigned steps;  // two-sweep steps so far
-    bool ok;
+    bool ok;  // (rows that are not a multiple of 16 bytes) no wait has run out
     // the unit
     T *out;
     int x0, ya, h, zb;
     bool own;
     J2Edge ed;
 
+    // Set once a wait of a block has run out for good.
+    __device__ __forceinline__ static int &dead() {
+        __shared__ int d;
+        return d;
+    }
     __device__ __forceinline__ void wait(uint64_t *b, unsigned parity) {
-        // after a timeout nothing waits any more and the next grid barrier ends the run
-        if (ok && !mbar_wait_bounded(b, parity, budget)) {
-            ok = false;
-            if (atomicCAS(&bar->error, 0, 1) == 0) bar->where = (int)steps;
+        if (!VEC) {
+            // after a timeout nothing waits any more and the next grid barrier, before which the
+            // producer's cp.async have landed, ends the run
+            if (ok && !mbar_wait_bounded(b, parity, budget)) {
+                ok = false;
+                if (atomicCAS(&bar->error, 0, 1) == 0) bar->where = (int)steps;
+            }
+            return;
+        }
+        // A wait beyond its budget is an error, which ends the run at the next grid barrier, but goes
+        // on (bounded): no stage may be handed on, and the block may not give up its shared memory,
+        // while a tensor copy into it is in flight.  All of it in one loop and without a flag in a
+        // register: this stands fifteen times in the march, where instructions and registers are
+        // short (512^3, 100 sweeps, ms: an `ok` that every wait tests, as above, FP64 27.75, FP32 17.5; this
+        // 26.8 and 17.3; waiting on in a second loop 28.1 and 19.8, in a call 28.9 and 17.5).
+        if (mbar_try_wait(b, parity)) return;
+        const unsigned long long t0 = global_ns();
+        while (!mbar_try_wait(b, parity)) {
+            const unsigned long long t = global_ns() - t0;
+            if (t <= budget) continue;
+            *(volatile int *)&bar->where = (int)steps;
+            *(volatile int *)&bar->error = 1;
+            if (t > budget + DRAIN_NS || *(volatile int *)&dead()) {
+                dead() = 1;
+                return;
+            }
         }
     }
     __device__ __forceinline__ static void unpack(const float4 &t, Row &v) {
@@ -271,13 +298,6 @@ struct J3PairWarp {
     }
 };
 
-// Waits (bounded) until the last copy into each of the `filled` stages has landed: those
-// before `slot` were filled in this turn around the ring, the others in the one before.  A call of
-// its own: inlined, it costs the consumers registers that spill.
-static __device__ __noinline__ void j3p_drain(uint64_t *full, int filled, int slot, unsigned turn, unsigned long long ns) {
-    for (int i = 0; i < filled; ++i) mbar_wait_bounded(full + i, i < slot ? turn : turn ^ 1, ns > DRAIN_NS ? ns : DRAIN_NS);
-}
-
 template <typename T, int CW, int R, int S, bool PY, bool VEC>
 __global__ void __launch_bounds__(32 * (CW + 1), 1)
     j3d_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, T *g0, T *g1,
@@ -314,6 +334,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1)
             mbar_init(&w.empty[i], CW);
         }
         for (int i = 0; i < 4 * CW; ++i) mbar_init(&w.ready[i], 1);
+        w.dead() = 0;
         mbar_fence_init();
     }
     __syncthreads();
@@ -343,7 +364,6 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1)
             const int h = 1 + (int)((long long)(ty + 1) * PR / nty) - ya;
             const int zb = 1 + ch * zchunk, ze = min(PZ + 1, zb + zchunk);
             if (producer) {
-                if (!w.ok) break;  // (alike in all lanes)
                 // window row l is grid row ya - 2 + l; off-grid columns read as 0
                 const bool on = x0 < nx;
                 const size_t pitch = on ? nx : 0;
@@ -352,13 +372,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1)
                 const CUtensorMap *map = in == g0 ? &map0 : &map1;
                 for (int s = zb - H; s < ze + H; ++s, w.next()) {
                     const int slot = w.slot;
-                    if (filled >= S) {
-                        w.wait(&w.empty[slot], w.turn ^ 1);
-                        // (landed long ago, unless a consumer ran out of budget and went on)
-                        w.wait(&w.full[slot], w.turn ^ 1);
-                    }
-                    // after a timeout no more copies: a stage may still be in use
-                    if (!(w.ok = __all_sync(J2_FULL, w.ok))) break;
+                    if (filled >= S) w.wait(&w.empty[slot], w.turn ^ 1);
                     filled = min(filled + 1, S);
                     int z = s;
                     if (site > 0) {  // ring of the planes 1 .. nz-2
@@ -429,13 +443,11 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1)
         }
         left -= pair ? 2 : 1;
         if (producer) cp_async_wait_all();
-        if (!grid_barrier(bar, gridDim.x, site)) break;
+        if (!grid_barrier(bar, gridDim.x, site)) return;
         T *t = in;
         in = out;
         out = t;
     }
-    // on an error exit the block keeps its shared memory until no copy into it is in flight
-    if (producer && w.lane == 0 && ld_relaxed_i32(&bar->error)) j3p_drain(w.full, filled, w.slot, w.turn, w.budget);
     // The result's halo cells (nothing above read any after the first sweep): full
     // rows of the planes 0 and nz-1, and with PY the rows 0 and ny-1 of the others.
     const int warps = gridDim.x * (CW + 1);

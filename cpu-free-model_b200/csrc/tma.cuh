@@ -59,8 +59,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
     return true;
 }
 
-// How long a block that leaves on an error waits for each of its copies still in
-// flight (at least; a wait's own budget may be far shorter than a copy).
+// How long a block with an error waits on for a copy still in flight (a wait's own budget
+// may be far shorter than a copy).
 constexpr unsigned long long DRAIN_NS = 1000000000ull;
 
 // Orders this thread's earlier generic-proxy accesses to the CTA's shared
