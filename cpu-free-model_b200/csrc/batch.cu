@@ -118,12 +118,26 @@ __device__ __forceinline__ float bt_apply32(const BtArgs &a, const BtSys &S, con
     return t;
 }
 
-// Sum of one partial slot over the system's tiles (fixed order).
+// Sum of one partial slot over the system's tiles (fixed order), block_sum's tree with the
+// last stage by one warp: where every warp adds the 32 warp sums for itself the FP64 kernel spills,
+// and 256 systems of up to 512^2 and 128^3 take 811 ms instead of 776 (mixed 645 instead of 597).
+// sm: 33 doubles.
 __device__ __forceinline__ double bt_sum(const BtArgs &a, const BtSys &S, int slot, double *sm) {
     const double *pp = a.part + S.poff + (long long)slot * S.ntiles;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double acc = 0.0;
     for (int i = threadIdx.x; i < S.ntiles; i += CG_TILE) acc += pp[i];
-    return block_sum(acc, sm);
+    acc = warp_xor_sum(acc);
+    if (lane == 0) sm[warp] = acc;
+    __syncthreads();
+    if (warp == 0) {
+        acc = warp_xor_sum(sm[lane]);
+        if (lane == 0) sm[32] = acc;
+    }
+    __syncthreads();
+    acc = sm[32];
+    __syncthreads();
+    return acc;
 }
 
 // r_i z_i for the <r, z> partials: the FP64 product, or the exact product

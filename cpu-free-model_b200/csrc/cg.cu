@@ -341,7 +341,7 @@ const void *solver_fn(int impl) {
     }
 }
 
-// HBM bytes of `iters` iterations: the operator data that the passes read plus the vector
+// Bytes of `iters` iterations: the operator data that the passes read plus the vector
 // passes of the method (8 B per FP64 entry read or written, 4 per FP32).  Row classes
 // replace column indices and, by value, the values by a byte per row (their tables stay
 // in L1); a system on chip is read once and its solution written once.

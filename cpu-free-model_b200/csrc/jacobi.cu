@@ -702,13 +702,13 @@ int setup_tma(cfm_jacobi *h, int var, int zchunk = 0) {
 // Two sweeps per pass (shape 12) where the two grids are well beyond L2, or so small that the
 // passes' latency and barriers are most of a sweep; between, one sweep per pass (shape
 // 0), which has no overlap to compute twice and runs from L2.  100 sweeps on B200, ms, one
-// sweep per pass against two.  FP64: 64^3 0.77 / 0.46, 128^3 (34 MB) 0.86 / 1.06, 192^3 (113 MB) 2.30
-// / 2.61, 224^3 (180 MB) 3.74 / 3.64, 250 x 250 x 256 (256 MB) 4.81 / 4.73, 256^3 (268 MB) 5.26 / 5.42,
-// 264^3 (294 MB) 5.71 / 5.59, 288^3 (382 MB) 7.38 / 5.73, 384^3 18.1 / 12.6, 512^3 41.4 / 27.7.  FP32: 128^3
-// (17 MB) 0.82 / 0.66, 256^3 (134 MB) 3.19 / 4.33, 304^3 (225 MB) 4.72 / 4.85, 320^3 (262 MB) 6.04 / 5.41,
-// 400^3 (512 MB) 12.2 / 12.6, 512^3 23.5 / 17.5.  So between 180 and 330 MB they are within 4% of one
+// sweep per pass against two.  FP64: 64^3 0.77 / 0.44, 128^3 (34 MB) 0.86 / 1.06, 192^3 (113 MB) 2.28
+// / 2.63, 224^3 (180 MB) 3.74 / 3.66, 250 x 250 x 256 (256 MB) 4.81 / 4.74, 256^3 (268 MB) 5.29 / 5.31,
+// 264^3 (294 MB) 5.70 / 5.56, 288^3 (382 MB) 7.34 / 5.61, 384^3 18.2 / 12.4, 512^3 41.1 / 26.9.  FP32: 128^3
+// (17 MB) 0.82 / 0.66, 256^3 (134 MB) 3.17 / 4.15, 304^3 (225 MB) 4.71 / 4.86, 320^3 (262 MB) 6.03 / 5.30,
+// 400^3 (512 MB) 12.1 / 12.5, 512^3 23.6 / 17.3.  So between 180 and 330 MB they are within 4% of one
 // another in FP64, and where the tiles' last column hangs over the grid (400^3) beyond it; the line lies
-// where FP32 gains 10%.  Rows that are not a multiple of 16 bytes have no one-sweep shape.
+// where FP32 gains 12%.  Rows that are not a multiple of 16 bytes have no one-sweep shape.
 // CFM_J3D_TMA_VARIANT (an index into the table) overrides.
 int default_tma_variant(cfm_jacobi *h) {
     int n = 0;
@@ -813,7 +813,9 @@ bool j2_tiling(int nx, int ny, int rows, int K, int blocks, J2Tiling *t) {
 // 32 warps; 2.7 us per exchange).  On chip against streaming: 1024^2 FP64 1.5 against 2.9
 // us per sweep, 1500^2 FP32 1.5 against 3.0, 1100^2 FP64 with K = 4 (the least) 2.7
 // against 2.7.  Resident handles keep to blocks of 1024 threads where those cover the
-// grid (cfm_jacobi_launch_shape's sign of an on-chip run).
+// grid: callers take cfm_jacobi_launch_shape's 1024 for the resident kernel.  That costs 3 to 4%
+// (100 sweeps of 1024^2 FP64 180 us resident, 173 persistent); of the 32-warp shapes only the FP64 one
+// with four rows serves other handles.
 int plan_j2(cfm_jacobi *h) {
     const cfm_jacobi_params &p = h->p;
     J2Plan best;
@@ -1092,12 +1094,11 @@ int launch_tma(cfm_jacobi *h, const TmaConfig &c, int count, int *launches) {
 // The pipeline shape of a run of niter sweeps.  Beside a two-sweep shape of the default
 // rule, short runs of grids that are not far beyond L2 take the one-sweep shape: the first
 // sweep and an odd rest have a pass to themselves, which the two-sweep kernel makes slower
-// (one sweep per pass against two, us on B200: one and two sweeps of 256^3 FP64 (268 MB) 64 / 80 and 120
-// / 172, 320^3 FP64 (524 MB) 119 / 114 and 226 / 261, 384^3 FP64 (906 MB) 193 / 179 and 377 / 378,
-// 100^3 FP64 (16 MB) 18 / 21 and 26 / 31, 64^3 FP64 (4 MB) 18 / 16 and 25 / 22; eight sweeps of 256^3
-// FP64 452 / 496, 272^3 FP64 (322 MB) 480 / 528, 288^3 FP64 (382 MB) 599 / 506, 100 sweeps of those 5.3 /
-// 5.4, 5.9 / 5.9 and 7.4 / 5.7 ms; in FP32 beyond 250 MB neither is ahead throughout: two sweeps of
-// 320^3 137 / 149, of 360^3 190 / 170).
+// (one sweep per pass against two, us on B200: one and two sweeps of 256^3 FP64 (268 MB) 61 / 78 and 114
+// / 167, 320^3 FP64 (524 MB) 118 / 111 and 225 / 254, 384^3 FP64 (906 MB) 192 / 175 and 373 / 368,
+// 100^3 FP64 (16 MB) 18 / 21 and 27 / 30, 64^3 FP64 (4 MB) 18 / 16 and 24 / 23; eight sweeps of 256^3
+// FP64 436 / 482, 272^3 FP64 (322 MB) 482 / 517, 288^3 FP64 (382 MB) 605 / 492; in FP32 beyond 250 MB neither
+// is ahead throughout: two sweeps of 320^3 131 / 145, of 360^3 181 / 165).
 const TmaConfig &tma_shape(const cfm_jacobi *h, int niter) {
     if (h->tc.sweeps == 1 || !h->tail.ok) return h->tc;
     if (h->dataflow) return h->tail;

@@ -149,8 +149,8 @@ struct TileSums {
 __device__ __forceinline__ double xprod(float a, float b) { return __dmul_rn((double)a, (double)b); }
 
 // U of the block's tiles per step (t0 + u gridDim.x, u < U), the FP32
-// passes' form of the tile pairs.  U = 2 measured best on 128^3 Poisson
-// (4: 22.3 ms mixed against 19.6 ms).
+// passes' form of the tile pairs.  Mixed, us per iteration on B200 for U = 1, 2, 4: 128^3
+// 7-point with row classes 34.2 / 32.7 / 35.7, renumbered so that it has none 58.9 / 51.5 / 62.4.
 constexpr int INNER_U = 2;
 template <int U>
 struct TileGroup {
@@ -173,9 +173,9 @@ struct Vals32 {
 
 // ------------------------------------------------------------- operators
 // CSR entries per row whose loads a thread issues together (CsrOp::apply2_t,
-// the FP64 passes): 4 and 8 both took standard CG on 128^3 Poisson from
-// 26.4 to 25.5 ms (bit-identical); the same form in the FP32 passes was no
-// faster (20.1-20.9 against 19.9-20.2 ms), so those keep one entry per step.
+// the FP64 passes).  Standard CG on 128^3 7-point renumbered so that it has no row
+// classes, us per iteration for 1, 4, 8: 73.3 / 71.4 / 71.1 (bit-identical); the same form
+// in the FP32 passes was no faster, so those keep one entry per step.
 constexpr int CSR_Q = 4;
 struct CsrOp {
     static constexpr bool ROW_FIRST = false;  // phase_pipe_step (its registers would spill)

@@ -84,9 +84,10 @@ typedef struct cfm_stats {
     long long iterations; /* sweeps (Jacobi) or CG iterations performed */
     double lups;          /* lattice-point updates (Jacobi) */
     double glups;         /* lups / seconds / 1e9 */
-    double bytes;         /* HBM bytes that the solve's passes over its data read and write, each word once
-                             per pass (Jacobi: 16 B per interior point and pass in FP64, 8 in FP32, where a
-                             pass may take several sweeps and a grid or system on chip is one pass) */
+    double bytes;         /* bytes of device memory that the solve's passes over its data read and write, each
+                             word once per pass, L2 hits included (Jacobi: 16 B per interior point and pass in
+                             FP64, 8 in FP32, where a pass may take several sweeps and a grid or system on
+                             chip is one pass) */
     double gbs;           /* bytes / seconds / 1e9 */
     double residual;      /* CG: final FP64 true relative residual ||b-Ax||/||b|| */
     double h2d_bytes;     /* host->device bytes copied inside the call */
